@@ -89,6 +89,17 @@ struct GateProgDev {
   uint32_t group;              // cells per group G = 32 / W, W = words per fused tile
 };
 
+// A flat gate program on the device (flatprog.h).
+struct FlatProgDev {
+  const uint4* stream;         // [entry][32] FlatLane
+  const uint32_t* warp_begin;  // [warps + 1]
+  const uint32_t* warp_tail;   // [warps]
+  const uint32_t* src_net;
+  const uint32_t* src_slot;
+  const GateRegDev* commit;    // rows (kFlatConst0/1: a constant)
+  uint32_t n_src, n_commit, n_slots;
+};
+
 struct GateRunDev {
   unsigned long long cycles, seed;
   uint32_t n_stim;
@@ -106,6 +117,7 @@ struct GateRunDev {
   const GateForceDev* forces;
   uint32_t has_forces;
   uint32_t final_settle;
+  uint32_t flat_serial;       // flat kernel: stimulus may only be stored after the record (a stimulated net is recorded)
   uint32_t* nets;             // [rows][words_pad]
   uint32_t* err;              // device status word
   unsigned long long cycle_base;  // absolute cycle of the launch's first cycle (stimulus, records)

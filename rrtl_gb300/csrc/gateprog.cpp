@@ -626,8 +626,12 @@ GateProgram build_gate_program(const MachineProgram& mp, uint32_t tile_words) {
     last_use[r.d_net] = kEnd;
     last_use[r.rst_net] = kEnd;
   }
+  gp.net_is_output.assign(gp.n_nets, 0);
   for (uint32_t s = 0; s < ns; ++s)
-    if (P.signals[s].kind == PSK::Output) last_use[2 + s] = kEnd;
+    if (P.signals[s].kind == PSK::Output) {
+      last_use[2 + s] = kEnd;
+      gp.net_is_output[2 + s] = 1;
+    }
   auto end_live = [&](uint32_t n) { return std::max(last_use[n], gp.net_level[n]) >= kEnd; };
 
   // ---- on-chip slots

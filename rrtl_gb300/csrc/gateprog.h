@@ -83,6 +83,7 @@ struct GateProgram {
   std::vector<GateReg> regs;
   // on-chip slots
   std::vector<int32_t> net_slot;  // -1: not resident
+  std::vector<uint8_t> net_is_output;   // net of an output signal
   std::vector<uint8_t> net_end_live;  // holds its value in its slot when the cycle's settle ends
   uint32_t n_slots = 0;           // including the scratch slot (slot 0)
   std::vector<uint32_t> source_nets;  // nets loaded into slots at tile start (and written back)

@@ -21,6 +21,8 @@ size_t gate_queue_static_smem();
 cudaError_t launch_gate_queue(const GateQueueDev& Q, uint32_t grid, size_t smem, cudaStream_t st);
 int gate_fused_ctas_per_sm(const GateProgDev& P, size_t smem);
 cudaError_t launch_gate_fused(const GateProgDev& P, const GateRunDev& R, uint32_t grid, size_t smem, cudaStream_t st);
+cudaError_t launch_gate_flat(uint32_t V, uint32_t N, uint32_t Q, const FlatProgDev& P, const GateRunDev& R, uint32_t grid,
+                             cudaStream_t st);
 cudaError_t launch_gate_plain(const GateProgDev& P, const GateRunDev& R, uint64_t c, int phase, cudaStream_t st);
 cudaError_t launch_word(const WordProgDev& P, const WordRunDev& R, bool smem_slots, cudaStream_t st);
 cudaError_t word_prepare(size_t smem);
@@ -274,6 +276,69 @@ GateVariant* gate_variant(rrtl_design* d, uint32_t W) {
   return d->gvar[li].get();
 }
 
+// Build and upload the flat program of row width V for Q warp sets.
+FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q) {
+  std::lock_guard<std::mutex> lk(d->gvar_mu);
+  std::unique_ptr<FlatVariant>& slot = d->fvar[log2_words(V)][Q - 1];
+  if (slot) return slot.get();
+  auto v = std::make_unique<FlatVariant>();
+  const GateProgram& gp = d->gp();
+  const uint32_t top = V == 4 ? kFlatMaxVectors : Q;
+  auto fit = [&](uint32_t slots) {  // vectors whose planes hold `slots` rows
+    uint32_t n = 0;
+    for (uint32_t k = 1; k <= top; ++k)
+      if ((size_t)slots * V * 4 <= flat_plane_bytes(k)) n = k;
+    return slots <= kMaxSlots && d->ctx->max_smem >= kFlatSmem ? n : 0u;
+  };
+  FlatOptions o;
+  o.warps = kFlatComputeThreads / 32 / Q;
+  v->fp = build_flat_program(gp, V, o);
+  v->max_n = fit(v->fp.n_slots);
+  if (v->max_n < top) {
+    // a little over the next step: trade write conflicts for a shorter slot array
+    o.max_slots = flat_plane_bytes(v->max_n + 1) / (V * 4);
+    if (v->fp.n_slots <= o.max_slots + o.max_slots / 8) {
+      FlatProgram f2 = build_flat_program(gp, V, o);
+      if (fit(f2.n_slots) > v->max_n) {
+        v->fp = std::move(f2);
+        v->max_n = fit(v->fp.n_slots);
+      }
+    }
+  }
+  const FlatProgram& fp = v->fp;
+  if (v->max_n) {
+    std::vector<uint32_t> src_slot, warps(fp.warp_begin);
+    for (uint32_t n : fp.source_nets) src_slot.push_back((uint32_t)fp.net_slot[n]);
+    warps.insert(warps.end(), fp.warp_tail.begin(), fp.warp_tail.end());
+    auto row = [&](uint32_t net) {
+      return net == kNetConst0 ? kFlatConst0 : net == kNetConst1 ? kFlatConst1 : (uint32_t)fp.net_slot[net];
+    };
+    std::vector<GateRegDev> commit;
+    for (uint32_t k : fp.commit) {
+      const GateReg& r = gp.regs[k];
+      const uint32_t fl = (r.has_reset ? 1u : 0u) | (r.active_low ? 2u : 0u) | (r.reset_value ? 4u : 0u);
+      commit.push_back(GateRegDev{row(r.q_net), row(r.d_net), r.has_reset ? row(r.rst_net) : kFlatConst0, fl});
+    }
+    upload(v->d_stream, fp.stream);
+    upload(v->d_warps, warps);
+    upload(v->d_src_net, fp.source_nets);
+    upload(v->d_src_slot, src_slot);
+    upload(v->d_commit, commit);
+    FlatProgDev& P = v->dev;
+    P.stream = v->d_stream.as<uint4>();
+    P.warp_begin = v->d_warps.as<uint32_t>();
+    P.warp_tail = P.warp_begin + fp.warps + 1;
+    P.src_net = v->d_src_net.as<uint32_t>();
+    P.src_slot = v->d_src_slot.as<uint32_t>();
+    P.commit = v->d_commit.as<GateRegDev>();
+    P.n_src = (uint32_t)fp.source_nets.size();
+    P.n_commit = (uint32_t)commit.size();
+    P.n_slots = fp.n_slots;
+  }
+  slot = std::move(v);
+  return slot.get();
+}
+
 // Load-time variant: the widest tile whose slots fit on chip. Slot counts
 // barely depend on W, so a miss at W = 8 predicts the width that fits.
 void build_gate_variants(rrtl_design* d) {
@@ -331,6 +396,63 @@ uint32_t choose_tile_words(rrtl_design* d, uint32_t words) {
     }
   }
   return best_w;
+}
+
+// Row width V, vectors per warp set N and warp sets Q of a flat run over
+// `words` 32-lane words (V = 0: the design does not fit), or those of an
+// explicit tile width. RRTL_FLAT=0 keeps the fused kernel and RRTL_FLAT=VNQ
+// forces a shape (A/B switches).
+//
+// The cost of a tile-cycle in SM clocks was measured on the 50,000-gate
+// netlist (41 levels, 860 entries, 17,700 wavefronts per 4-word vector), one
+// wave of tiles: 25.1k at one-word rows, 29.0k at two, and 37.5k / 56.4k /
+// 79.0k / 98.2k for one to four 4-word vectors (four of them as two warp sets
+// of two: 100.1k as one set). So a tile costs about 250 clocks a level, 10 an
+// entry and 1.2 a wavefront, and wide tiles pay until the last round of tiles
+// leaves most SMs idle.
+struct FlatShape {
+  uint32_t V = 0, N = 1, Q = 1;
+};
+FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w) {
+  FlatShape s;
+  auto checked = [&](FlatShape x) {
+    if (x.V && flat_variant(d, x.V, x.Q)->max_n < x.N * x.Q) x.V = 0;
+    return x;
+  };
+  const char* env = getenv("RRTL_FLAT");
+  if (env && env[0] == '0') return s;
+  if (env && strlen(env) == 3) {
+    s.V = (uint32_t)(env[0] - '0');
+    s.N = (uint32_t)(env[1] - '0');
+    s.Q = (uint32_t)(env[2] - '0');
+    return checked(s);
+  }
+  if (explicit_w) {
+    s.V = std::min(explicit_w, 4u);
+    s.N = explicit_w / s.V;
+    return checked(s);
+  }
+  // the widest rows that fit; packing leaves fewer live nets than the fused program's slots
+  uint32_t top = 0;
+  for (uint32_t V = 4; V >= 1 && !top; V /= 2)
+    if ((size_t)d->gp().n_slots * V * 4 <= flat_plane_bytes(1) / 4 * 5 && flat_variant(d, V, 1)->max_n) top = V;
+  if (!top) return s;
+  const FlatVariant* v = flat_variant(d, top, 1);
+  const FlatProgram& fp = v->fp;
+  const double vec4 = (double)fp.wavefronts * (top == 4 ? 1.0 : top == 2 ? 1.85 : 3.4);  // wavefronts of 4-word rows
+  const FlatShape shapes[] = {{4, 2, 2}, {4, 3, 1}, {4, 2, 1}, {4, 1, 1}, {2, 1, 1}, {1, 1, 1}};
+  double best = INFINITY;
+  for (const FlatShape& x : shapes) {
+    if (x.V > top || (x.V == 4 && x.N * x.Q > v->max_n)) continue;
+    const double work = vec4 * (x.V == 4 ? 1.2 * x.N * x.Q : x.V == 2 ? 0.58 : 0.36);
+    const double rounds = std::ceil(std::ceil((double)words / (x.V * x.N * x.Q)) / d->ctx->sm_count);
+    const double t = rounds * (fp.n_levels * 250.0 + fp.n_entries * 10.0 + work);
+    if (t < best) {
+      best = t;
+      s = x;
+    }
+  }
+  return checked(s);
 }
 
 void upload_word_program(rrtl_design* d) {
@@ -436,11 +558,29 @@ void invalidate_forces(rrtl_batch* b) {
 // context stream. `want_fused` asks for the fused path (it falls back to the
 // plain path when a recorded net does not stay on chip to the end of a cycle).
 GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool want_fused,
-                          const CheckTables* chk) {
+                          const CheckTables* chk, bool want_flat) {
   rrtl_design* d = b->d;
   cudaStream_t st = d->ctx->stream;
   GatePrepared g;
-  const uint32_t W = want_fused ? (b->tile_words ? b->tile_words : choose_tile_words(d, b->words)) : 0;
+  if (want_flat && want_fused && run.cycles >= kFlatMinCycles && b->faults.empty() && d->gate_w_max) {
+    uint32_t ew = b->tile_words;
+    auto tuned = d->tuned_w.find(lane_bucket(b->words));
+    if (!ew && tuned != d->tuned_w.end() && tuned->second != kTunedCompiled) ew = tuned->second;
+    const FlatShape fs = choose_flat(d, b->words, ew);
+    bool ok = fs.V != 0;
+    for (uint32_t i = 0; ok && i < run.n_record; ++i)
+      ok = run.record[i] < d->gp().signal_net.size() &&
+           flat_variant(d, fs.V, fs.Q)->fp.recordable[d->gp().signal_net[run.record[i]]];
+    if (ok) {
+      g.flat = flat_variant(d, fs.V, fs.Q);
+      g.flat_n = fs.N;
+      g.flat_q = fs.Q;
+    }
+  }
+  // (the fused kernel only closes a flat run: the variant built at load time does)
+  const uint32_t W = !want_fused ? 0
+                     : g.flat    ? d->gate_w_max
+                                 : (b->tile_words ? b->tile_words : choose_tile_words(d, b->words));
   GateVariant* v = W ? gate_variant(d, W) : d->gvar[d->gate_base].get();
   const GateProgram& gp = v->gp;
   bool fused = W && v->fused_ok;
@@ -459,12 +599,17 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   for (uint32_t i = 0; i < run.n_record; ++i) {
     signal_of(d, run.record[i]);
     uint32_t net = gp.signal_net[run.record[i]];
-    if (fused && !v->end_live[net]) fused = false;  // value not held to the end of the cycle: use the plain path
+    if (fused && !g.flat && !v->end_live[net]) fused = false;  // value not held to the end of the cycle: use the plain path
     rec.push_back(GateRecDev{0u, net});
   }
   if (fused) {
-    for (auto& r : rec) r.slot = (uint32_t)gp.net_slot[r.net];
-    for (auto& s : stim) s.slot = (uint32_t)gp.net_slot[s.net];
+    const std::vector<int32_t>& rows = g.flat ? g.flat->fp.net_slot : gp.net_slot;
+    for (auto& r : rec) r.slot = (uint32_t)rows[r.net];
+    for (auto& s : stim) s.slot = (uint32_t)rows[s.net];
+    if (g.flat)
+      for (auto& r : rec)
+        for (auto& s : stim)
+          if (r.net == s.net) g.R.flat_serial = 1;
   }
   REQUIRE(!(run.record_mode & (RRTL_REC_TRACE | RRTL_REC_HASH | RRTL_REC_DETECT)) || run.n_record > 0, RRTL_E_ARG,
           "E_GPU_RECORD: recording needs at least one signal");
@@ -548,6 +693,24 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   g.fused = fused;
   g.W = fused ? W : 0;
   return g;
+}
+
+// A flat run: the cycles on the flat kernel, then the closing settle, which
+// writes every signal back, on the fused kernel.
+void gate_flat_launch(rrtl_design* d, const GatePrepared& g, cudaStream_t st) {
+  const uint32_t V = g.flat->fp.V, W = V * g.flat_n * g.flat_q;
+  GateRunDev R = g.R;
+  R.n_tiles = (g.R.words_pad + W - 1) / W;
+  cuda_check(launch_gate_flat(V, g.flat_n, g.flat_q, g.flat->dev, R, std::min(R.n_tiles, d->ctx->sm_count), st),
+             "gate_flat_kernel");
+  GateRunDev C = g.R;
+  C.cycles = 0;
+  C.n_stim = 0;
+  C.n_rec = 0;
+  C.mode = 0;
+  C.n_tiles = g.R.words_pad / g.W;
+  const uint32_t grid = std::min<uint32_t>(C.n_tiles, d->ctx->sm_count * g.v->fused_ctas);
+  cuda_check(launch_gate_fused(g.v->gdev, C, grid, g.v->fused_smem, st), "gate_fused_kernel");
 }
 
 // Copy a prepared run's recorded outputs to the caller's host buffers.
@@ -641,18 +804,22 @@ void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckT
               bool force_compiled = false) {
   rrtl_design* d = b->d;
   cudaStream_t st = d->ctx->stream;
-  GatePrepared g = gate_prepare(b, run, device_ptrs, b->path == RRTL_PATH_FUSED, chk);
+  const bool compiled = b->path == RRTL_PATH_FUSED && b->faults.empty() &&
+                        (force_compiled || (b->tile_words == 0 && gate_jit_preferred(d, b->words)));
+  GatePrepared g = gate_prepare(b, run, device_ptrs, b->path == RRTL_PATH_FUSED, chk, !compiled);
   // the compiled gate kernel: automatic tile width, no stuck-at forces; built before the timed region
-  const JitKernel* J = nullptr;
-  if (b->path == RRTL_PATH_FUSED && !g.R.has_forces && (force_compiled || (b->tile_words == 0 && gate_jit_preferred(d, b->words))))
-    J = gate_jit_for_run(d, g.tables);
+  const JitKernel* J = compiled && !g.R.has_forces ? gate_jit_for_run(d, g.tables) : nullptr;
   // the fused kernel compiled for the design's truth-table classes, also built before the timed region
-  const JitKernel* F = !J && g.fused ? fused_jit_for(d, g.v) : nullptr;
+  const JitKernel* F = !J && g.fused && !g.flat ? fused_jit_for(d, g.v) : nullptr;
   Timer tm(b);
   if (J) {
     g.R.cycle_base = 0;
     cuda_check(launch_gate_jit(*J, g.R, st), "rrtl_gate_jit");
     g.W = 0;
+  } else if (g.flat && g.fused) {
+    gate_flat_launch(d, g, st);
+    g.W = g.flat->fp.V * g.flat_n * g.flat_q;
+    if (g.W > 8) g.W = g.W == 16 ? 8 : 4;  // several tiles of the widest documented width that divides them
   } else if (g.fused) {
     uint32_t grid = std::min<uint32_t>(g.R.n_tiles, d->ctx->sm_count * g.v->fused_ctas);
     if (F)

@@ -12,6 +12,7 @@
 
 #include "../../include/rrtl_cuda.h"
 #include "gate_dev.h"
+#include "flatprog.h"
 #include "gate_jit.h"
 #include "gateprog.h"
 #include "lower.h"
@@ -67,6 +68,14 @@ struct GateVariant {
   DevBuf d_srecs, d_pieces, d_src_net, d_src_slot, d_sregs, d_wb, d_grecs, d_lgb, d_gregs;
 };
 
+// The flat program for one row width V, with its device copy.
+struct FlatVariant {
+  FlatProgram fp;
+  FlatProgDev dev{};
+  uint32_t max_n = 0;  // vectors of V words that fit in shared memory, 0: none
+  DevBuf d_stream, d_warps, d_src_net, d_src_slot, d_commit;
+};
+
 // Per-tile, per-stage force table of a batch for one tile width.
 struct ForceTable {
   bool valid = false;
@@ -82,6 +91,9 @@ struct GatePrepared {
   GateRunTables tables;  // host copies of the run's stimulus and record tables
   bool fused = false;
   uint32_t W = 0;
+  // the flat kernel runs the cycles and the fused kernel the closing settle
+  FlatVariant* flat = nullptr;
+  uint32_t flat_n = 0, flat_q = 0;  // vectors per warp set, warp sets
   size_t trace_out_bytes = 0, hash_bytes = 0, det_bytes = 0;
   bool want_trace = false, want_hash = false, want_det = false;
 };
@@ -132,7 +144,7 @@ struct CheckTables {
 
 // Runtime internals shared by the C ABI and the serving loop.
 GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool want_fused,
-                          const CheckTables* chk = nullptr);
+                          const CheckTables* chk = nullptr, bool want_flat = false);
 void gate_copy_out(rrtl_batch* b, const GatePrepared& g, const rrtl_run& run);
 void gate_plain_launches(const GatePrepared& g, uint64_t cycles, cudaStream_t st, bool graph);
 WordPrepared word_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool start_settle,
@@ -212,6 +224,7 @@ struct rrtl_design {
   // gate engine: one program per fused tile width W (index log2 W), built on
   // demand; nets, levels and registers are the same in every variant
   std::unique_ptr<rrtl::GateVariant> gvar[4];
+  std::unique_ptr<rrtl::FlatVariant> fvar[3][2];  // flat programs by log2 V and warp sets - 1
   uint32_t gate_base = 3;   // log2 W of the variant built at load time
   uint32_t gate_w_max = 0;  // widest W whose slots fit on chip, 0 if none
   std::map<uint32_t, uint32_t> tuned_w;  // measured best W by lane bucket (ceil log2 of 32-lane words);

@@ -1,0 +1,111 @@
+"""The flat gate kernel at every shape against the bit-parallel oracle: ragged
+lane counts around its tiles, every record form, more stimulus and record
+words than its service threads hold in registers, registers left on the
+commit list, a recorded input, and runs split in two."""
+import numpy as np
+import pytest
+
+from oracle import binding as ob
+from rrtl_gb300 import sim
+from rrtl_gb300.workloads import gate_netlist, netlist_run_spec
+
+from .helpers import oracle_bp_run
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = {"111": 1, "211": 2, "411": 4, "421": 8, "431": 12, "422": 16}
+
+
+@pytest.fixture(scope="module")
+def wide(engine):
+    """200 inputs and outputs: at 16 words a tile has 3,200 stimulus and record words."""
+    d, meta = gate_netlist(n_gates=4000, n_ff=300, n_pi=200, n_po=200, depth=9, seed=8)
+    js = d.to_json()
+    return sim.CompiledDesign(js, meta.top), meta, ob.OracleDesign(js, meta.top)
+
+
+def _ref(od, lanes, cycles, seed, stim, rec, mode, **kw):
+    return oracle_bp_run(od, lanes, cycles, seed, [(od.signal(n), k, p) for n, k, p in stim],
+                         [od.signal(r) for r in rec], mode, **kw)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("lanes", [1, 500, 32 * 16 * 3 + 7])
+def test_shapes_equal_the_oracle(wide, monkeypatch, shape, lanes):
+    cd, meta, od = wide
+    monkeypatch.setenv("RRTL_FLAT", shape)
+    stim, rec = netlist_run_spec(meta)
+    mode = sim.REC_TRACE | sim.REC_HASH | sim.REC_DETECT
+    g = sim.GpuBatchSimulator(cd, lanes=lanes)
+    res = g.run(13, seed=5, stim=stim, record=rec, mode=mode, lane_base=64)
+    assert g.tile_words == {12: 4, 16: 8}.get(SHAPES[shape], SHAPES[shape])
+    ref = _ref(od, lanes, 13, 5, stim, rec, mode, lane_base=64)
+    for k in ("trace", "hash", "detect"):
+        assert np.array_equal(res[k], ref[k]), k
+    ref["sim"].settle()
+    for n in meta.regs[::17] + meta.gate_names[::101] + meta.outputs[::9]:
+        assert np.array_equal(g.get_signal_bits(n), ref["sim"].get_bits(od.signal(n))), n
+
+
+@pytest.mark.parametrize("shape", ["111", "421", "422"])
+def test_trace_input_and_recorded_input(wide, monkeypatch, shape):
+    """Stimulus from a trace; a recorded net that is itself stimulated."""
+    cd, meta, od = wide
+    monkeypatch.setenv("RRTL_FLAT", shape)
+    lanes, cycles = 300, 11
+    words = (lanes + 31) // 32
+    tr = np.random.default_rng(4).integers(0, 1 << 32, (cycles, len(meta.inputs), words), dtype=np.uint32)
+    stim = [(meta.rst, sim.STIM_PULSE, 1)] + [(p, sim.STIM_TRACE, i) for i, p in enumerate(meta.inputs)]
+    rec = meta.outputs[:40] + meta.inputs[:5]
+    g = sim.GpuBatchSimulator(cd, lanes=lanes)
+    res = g.run(cycles, seed=1, stim=stim, record=rec, mode=sim.REC_TRACE | sim.REC_HASH, input_trace=tr)
+    assert g.tile_words == {12: 4, 16: 8}.get(SHAPES[shape], SHAPES[shape])
+    ref = _ref(od, lanes, cycles, 1, stim, rec, 3, input_trace=tr)
+    assert np.array_equal(res["trace"], ref["trace"]) and np.array_equal(res["hash"], ref["hash"])
+
+
+@pytest.mark.parametrize("shape", ["211", "422"])
+def test_runs_continue_from_the_state_they_leave(wide, monkeypatch, shape):
+    cd, meta, od = wide
+    monkeypatch.setenv("RRTL_FLAT", shape)
+    stim, rec = netlist_run_spec(meta)
+    hold = [(meta.rst, sim.STIM_CONST, 0)]  # inputs keep the values the first run left
+    g = sim.GpuBatchSimulator(cd, lanes=700)
+    a = g.run(6, seed=2, stim=stim, record=rec, mode=sim.REC_HASH)["hash"]
+    b = g.run(7, seed=2, stim=hold, record=rec, mode=sim.REC_HASH)["hash"]
+    monkeypatch.setenv("RRTL_FLAT", "0")
+    f = sim.GpuBatchSimulator(cd, lanes=700)
+    assert np.array_equal(a, f.run(6, seed=2, stim=stim, record=rec, mode=sim.REC_HASH)["hash"])
+    assert np.array_equal(b, f.run(7, seed=2, stim=hold, record=rec, mode=sim.REC_HASH)["hash"])
+    for n in meta.regs[::29] + meta.inputs[::31] + meta.gate_names[::211]:
+        assert np.array_equal(g.get_signal_bits(n), f.get_signal_bits(n)), n
+
+
+@pytest.mark.parametrize("shape", ["111", "411", "422"])
+def test_registers_on_the_commit_list(engine, monkeypatch, shape):
+    """A shift chain is longer than the levels, so part of it commits after them."""
+    from rrtl_gb300.builder import Design, mux, uint
+
+    d = Design()
+    m = d.module("Chain")
+    clk, rst, en, x = (m.input(n, uint(1)) for n in ("clk", "rst", "en", "x"))
+    regs = [m.reg(f"r{k}", uint(1)) for k in range(260)]
+    for k, r in enumerate(regs):
+        m.clock(r, clk)
+        if k % 3:
+            m.reset(r, rst, k % 2)
+        m.next(r, mux(en, regs[k - 1] if k else x, r))
+    for k in range(4):
+        o = m.output(f"o{k}", uint(1))
+        m.assign(o, regs[50 * k + 9] ^ regs[259])
+    js = d.to_json()
+    cd, od = sim.CompiledDesign(js, "Chain"), ob.OracleDesign(js, "Chain")
+    monkeypatch.setenv("RRTL_FLAT", shape)
+    monkeypatch.setenv("RRTL_GATE_JIT", "0")
+    stim = [("clk", sim.STIM_CONST, 1), ("rst", sim.STIM_PULSE, 2), ("en", sim.STIM_RANDOM, 1), ("x", sim.STIM_RANDOM, 2)]
+    rec = [f"o{k}" for k in range(4)]
+    g = sim.GpuBatchSimulator(cd, lanes=1000)
+    res = g.run(60, seed=9, stim=stim, record=rec, mode=3)
+    assert g.tile_words != 0
+    ref = _ref(od, 1000, 60, 9, stim, rec, 3)
+    assert np.array_equal(res["trace"], ref["trace"]) and np.array_equal(res["hash"], ref["hash"])
