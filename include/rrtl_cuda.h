@@ -552,8 +552,7 @@ rrtl_status rrtl_gate_jit_emit(const char* json, size_t len, const char* top, co
 
 /* The fused gate kernel compiled for one design (fused path of
  * rrtl_batch_run on the gate engine, for the runs the flat gate kernel does
- * not take: stuck-at faults, fewer than four cycles, designs whose rows do
- * not fit its layout): the generic kernel's code with a run
+ * not take: fewer than four cycles, designs whose rows do not fit its layout): the generic kernel's code with a run
  * dispatch over only the truth-table classes the design's cells use, which
  * leaves room for a split barrier between pieces in runs without stuck-at
  * forces (about 10% faster on a 50k-gate netlist: 11 of 80 classes). Built on the first such run of a tile width and cached with the

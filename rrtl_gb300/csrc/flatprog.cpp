@@ -107,8 +107,12 @@ struct Logic {
   std::vector<uint8_t> root;     // net must be in its own row at the end of a cycle
   std::vector<uint32_t> commit;  // registers left on the commit list
   uint32_t n_levels = 0;
+  bool observe = false;
 
   explicit Logic(const GateProgram& g) : gp(g) {}
+
+  // A net whose row nothing but its readers sees.
+  bool hidden(uint32_t net) const { return !(observe && gp.net_signal[net] >= 0); }
 
   void collect() {
     for (const GateCell& c : gp.cells) {
@@ -158,7 +162,7 @@ struct Logic {
       for (int k = 0; k < y.n;) {
         const int32_t x = cell_of[y.in[k]];
         FlatCell z;
-        if (x >= 0 && cells[x].n <= 1 && compose(y, k, cells[x], &z)) {
+        if (x >= 0 && cells[x].n <= 1 && hidden(cells[x].out) && compose(y, k, cells[x], &z)) {
           y = z;
           k = 0;
         } else {
@@ -177,7 +181,7 @@ struct Logic {
         FlatCell bz;
         for (int k = 0; k < y.n; ++k) {
           const int32_t x = cell_of[y.in[k]];
-          if (x < 0 || root[cells[x].out] || f[cells[x].out] != 1) continue;
+          if (x < 0 || root[cells[x].out] || f[cells[x].out] != 1 || !hidden(cells[x].out)) continue;
           FlatCell z;
           if (compose(y, k, cells[x], &z) && (best < 0 || z.n < bz.n)) {
             best = k;
@@ -243,7 +247,8 @@ struct Logic {
       const bool is_out = gp.net_is_output[g.d_net];
       FlatCell next;
       bool own = false;
-      if (dc >= 0 && alive[dc] && d_uses[g.d_net] == 1 && f[g.d_net] == 0 && !is_rst[g.d_net] && !is_out) {
+      if (dc >= 0 && alive[dc] && d_uses[g.d_net] == 1 && f[g.d_net] == 0 && !is_rst[g.d_net] && !is_out &&
+          hidden(g.d_net)) {
         next = cells[dc];
         own = add_reset(g, &next);
       }
@@ -609,6 +614,7 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
   fp.V = V;
   const uint32_t G = fp.G = 32 / V, warps = fp.warps = opt.warps;
   Logic lg(gp);
+  lg.observe = opt.observe;
   lg.collect();
   if (opt.pack) lg.pack();
   else lg.drop_dead();
@@ -751,6 +757,8 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
   const bool tight = opt.max_slots != 0;
 
   // ---- levels: group, place, schedule
+  fp.net_level.assign(gp.n_nets, -1);
+  fp.net_warp.assign(gp.n_nets, 0);
   Grouper grouper{G, cells, slot};
   std::vector<std::vector<FlatLane>> streams(warps);
   std::vector<uint32_t> last_level(warps, 0);
@@ -809,7 +817,8 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
     // entries of this level: V groups fill a warp's lanes
     struct Entry {
       std::vector<FlatLane> lanes;
-      double cost;
+      std::vector<uint32_t> outs;  // nets written
+      double cost = 0;
     };
     std::vector<Entry> es;
     auto lane_fill = [&](const std::vector<Group>& gs, size_t g0, auto&& put) {
@@ -838,9 +847,14 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
         }
       }
     };
+    auto outs_of = [&](Entry& e, const std::vector<Group>& gs, size_t g0, size_t n) {
+      for (size_t g = g0; g < std::min(gs.size(), g0 + n); ++g)
+        for (uint32_t ci : gs[g].cells) e.outs.push_back(cells[ci].out);
+    };
     for (size_t g = 0; g < g2.size(); g += 2 * V) {
       Entry e;
       e.lanes.resize(32);
+      outs_of(e, g2, g, 2 * V);
       lane_fill(g2, g, [&](uint32_t l, uint32_t a, uint32_t b, uint32_t, uint32_t o, uint8_t lut) {
         e.lanes[l].x = a | (b << 16);
         e.lanes[l].y = o | two_meta(lut);
@@ -855,6 +869,7 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
     for (size_t g = 0; g < g3.size(); g += V) {
       Entry e;
       e.lanes.resize(32);
+      outs_of(e, g3, g, V);
       lane_fill(g3, g, [&](uint32_t l, uint32_t a, uint32_t b, uint32_t c, uint32_t o, uint8_t lut) {
         e.lanes[l].x = a | (b << 16);
         e.lanes[l].y = o | kFlatDevThree;
@@ -876,6 +891,10 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
       }
       load[w] += e.cost;
       sched[w % 4] += e.cost;
+      for (uint32_t n : e.outs) {
+        fp.net_warp[n] = (uint8_t)w;
+        fp.net_level[n] = (int32_t)L;
+      }
       uint32_t syncs = L - last_level[w];
       last_level[w] = L;
       for (; syncs > 1; --syncs) push_idle(streams[w], kFlatDevSync);  // levels in which the warp has no entry

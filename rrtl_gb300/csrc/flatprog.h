@@ -10,7 +10,8 @@
 //     observed, so inverters and buffers are folded into their readers and a
 //     net with a single reader is folded into that reader where the result
 //     still has at most three inputs. (The closing settle, which writes every
-//     signal back, and runs with stuck-at forces use the unpacked program.)
+//     signal back, runs on the fused kernel; for runs with stuck-at forces
+//     FlatOptions::observe keeps a row for every signal.)
 //  2. Register folding: a cell that computes a register's next value writes
 //     the register's own row, with the synchronous reset in its function, at
 //     a level after every other read of the register. Registers for which
@@ -64,6 +65,8 @@ struct FlatProgram {
   std::vector<int32_t> net_slot;          // -1: not resident
   std::vector<uint8_t> recordable;        // net holds its value in its slot when the cycle's settle ends
   uint32_t n_slots = 0;                   // the first G are scratch rows of idle lanes
+  std::vector<int32_t> net_level;         // level a cell writes the net's row at, -1: none does
+  std::vector<uint8_t> net_warp;          // warp that does
   std::vector<uint32_t> source_nets;      // loaded at the start of a run, written back at its end
   std::vector<uint32_t> commit;           // GateProgram::regs indices not folded
   std::vector<FlatLane> stream;           // [entry][32 lanes]
@@ -77,6 +80,7 @@ struct FlatProgram {
 struct FlatOptions {
   bool pack = true;
   bool fold_regs = true;
+  bool observe = false;  // every signal keeps a row of its own (stuck-at forces act on any of them)
   uint32_t warps = kFlatComputeThreads / 32;
   uint32_t max_slots = 0;  // above this, a row is placed at any residue before the slot array grows (0: no limit)
 };

@@ -117,6 +117,13 @@ struct GateRunDev {
   const GateForceDev* forces;
   uint32_t has_forces;
   uint32_t final_settle;
+  // flat kernel: forces of comb nets by (tile, warp), those of a level together
+  // and levels ascending, and of registers by tile; x: byte offset from the
+  // slot array, y: mask, z: value, w: level
+  const uint32_t* flat_off;   // [n_tiles * warps + 1]
+  const uint4* flat_forces;
+  const uint32_t* flat_off0;  // [n_tiles + 1] into flat_forces0
+  const uint4* flat_forces0;
   uint32_t flat_serial;       // flat kernel: stimulus may only be stored after the record (a stimulated net is recorded)
   uint32_t* nets;             // [rows][words_pad]
   uint32_t* err;              // device status word

@@ -218,10 +218,58 @@ __device__ __forceinline__ void flat_one3(uint8_t* S, const uint4& r, uint32_t g
   }
 }
 
-// Cycles [c0, c0 + ncyc) of one tile (V * N words) of a run. Source nets are
+// Stuck-at forces of the comb nets one warp writes, applied by that warp when
+// it finished a level, before the level's barrier: no barrier of their own.
+// The list is sorted by level; each lane holds one force of a 32-force
+// window, which moves on once its last force's level is done.
+struct FlatForces {
+  const uint4* base;
+  uint32_t n, at, due;  // due: next level with a force
+  uint4 f;
+  __device__ __forceinline__ void load(uint32_t lane) {
+    f = at + lane < n ? __ldg(base + at + lane) : make_uint4(0u, 0u, 0u, 0xFFFFFFFFu);
+  }
+  __device__ __forceinline__ void begin(uint32_t lane, bool first) {
+    if (first || at) {
+      at = 0u;
+      load(lane);
+    }
+    due = __reduce_min_sync(0xFFFFFFFFu, f.w);
+  }
+  __device__ __forceinline__ void set(uint8_t* S, uint32_t level) const {
+    if (f.w == level) {
+      uint32_t& v = *reinterpret_cast<uint32_t*>(S + f.x);
+      v = (v & ~f.y) | (f.z & f.y);
+    }
+  }
+  // Before the level's barrier: the forces of `level`.
+  __device__ __forceinline__ void apply(uint8_t* S, uint32_t level, uint32_t lane) {
+    if (level != due) return;
+    __syncwarp();  // the warp's rows of this level are written
+    set(S, level);
+    while (at + 32u < n && last() <= level) {
+      at += 32u;
+      load(lane);
+      set(S, level);
+    }
+  }
+  // After it, where the other warps' row accesses cover the latency: the next level due.
+  __device__ __forceinline__ void advance(uint32_t level) {
+    if (level == due) due = __reduce_min_sync(0xFFFFFFFFu, f.w > level ? f.w : 0xFFFFFFFFu);
+  }
+  __device__ __forceinline__ uint32_t last() const { return __shfl_sync(0xFFFFFFFFu, f.w, 31); }
+};
+
+__device__ __forceinline__ void flat_bar_compute() {
+  __syncwarp();
+  asm volatile("bar.sync 4, %0;" ::"n"(kFlatComputeThreads) : "memory");
+}
+
+// Cycles [c0, c0 + ncyc) of one tile (V * N * Q words) of a run; F: with
+// stuck-at forces. Source nets are
 // read from and written back to the run's global rows; the caller settles the
 // other nets (the closing settle) afterwards.
-template <int V, int N, int Q>
+template <int V, int N, int Q, bool F>
 __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev& R, uint32_t tile, uint64_t c0,
                                           uint64_t ncyc, uint8_t* smem) {
   constexpr uint32_t W = V * N * Q;
@@ -250,7 +298,7 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
     dstate[16 + tid] = det;
   }
   __syncthreads();
-  const bool serial = P.n_commit != 0 || R.flat_serial;
+  const bool serial = F || P.n_commit != 0 || R.flat_serial;
   if (tid < kFlatComputeThreads) {
     constexpr uint32_t kSetWarps = kFlatComputeThreads / 32 / Q;
     const uint32_t set = Q == 1 ? 0u : tid / (kFlatComputeThreads / Q), warp = (tid >> 5) % kSetWarps;
@@ -258,11 +306,25 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
     const uint32_t begin = __ldg(P.warp_begin + warp), n = __ldg(P.warp_begin + warp + 1) - begin;
     const uint32_t tail = __ldg(P.warp_tail + warp);
     const uint4* const base = P.stream + (size_t)begin * 32u + lane;
+    FlatForces forces{};
+    uint32_t begin0 = 0, end0 = 0;  // forces of registers; the thread's first stays in registers
+    uint4 first0{};
+    if constexpr (F) {
+      const uint32_t k = tile * (Q * kSetWarps) + (tid >> 5);
+      forces.base = R.flat_forces + __ldg(R.flat_off + k);
+      forces.n = __ldg(R.flat_off + k + 1) - __ldg(R.flat_off + k);
+      forces.begin(lane, true);
+      begin0 = __ldg(R.flat_off0 + tile);
+      end0 = __ldg(R.flat_off0 + tile + 1);
+      if (begin0 + tid < end0) first0 = __ldg(R.flat_forces0 + begin0 + tid);
+    }
     uint4 q[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) q[d] = n ? flat_load_entry(base + d * 32) : make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();  // first cycle's stimulus in place
     for (uint64_t c = 0; c < ncyc; ++c) {
+      uint32_t level = 0;
+      if constexpr (F) forces.begin(lane, false);
       for (uint32_t e = 0; e < n; e += D) {
         const uint4* const ahead = base + (size_t)(e + D < n ? e + D : 0u) * 32u;
         uint4 nx[D];
@@ -272,14 +334,25 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
         for (int d = 0; d < D; ++d) {
           const uint4 r = q[d];
           const uint32_t go = r.y & kFlatDevSync;
+          if constexpr (F) {
+            if (go) forces.apply(S, level, lane);  // the same on every lane
+          }
           // (the vote makes the branch a warp-uniform one)
           if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, Q>(Sq, r, go, set);
           else flat_pair2<V, N, Q>(Sq, r, go, set);
+          if constexpr (F) {
+            if (go) forces.advance(level++);
+          }
         }
 #pragma unroll
         for (int d = 0; d < D; ++d) q[d] = nx[d];
       }
-      for (uint32_t k = tail; k; --k) flat_pass<Q>(1u, set);
+      for (uint32_t k = tail; k; --k) {
+        if constexpr (F) forces.apply(S, level, lane);
+        flat_pass<Q>(1u, set);
+        if constexpr (F) forces.advance(level++);
+      }
+      if constexpr (F) forces.apply(S, level, lane);
       __syncthreads();  // every level done
       if (serial) {
         // registers left on the commit list
@@ -293,6 +366,14 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
             d = (rr.w & 4u) ? d | m : d & ~m;
           }
           word_at(rr.x, ww) = d;
+        }
+        if constexpr (F) {
+          if (P.n_commit) flat_bar_compute();
+          for (uint32_t i = begin0 + tid; i < end0; i += kFlatComputeThreads) {
+            const uint4 f = i == begin0 + tid ? first0 : __ldg(R.flat_forces0 + i);
+            uint32_t& v = *reinterpret_cast<uint32_t*>(S + f.x);
+            v = (v & ~f.y) | (f.z & f.y);
+          }
         }
         __syncthreads();
       }

@@ -276,10 +276,11 @@ GateVariant* gate_variant(rrtl_design* d, uint32_t W) {
   return d->gvar[li].get();
 }
 
-// Build and upload the flat program of row width V for Q warp sets.
-FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q) {
+// Build and upload the flat program of row width V for Q warp sets; observe:
+// with a row for every signal (runs with stuck-at forces).
+FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe) {
   std::lock_guard<std::mutex> lk(d->gvar_mu);
-  std::unique_ptr<FlatVariant>& slot = d->fvar[log2_words(V)][Q - 1];
+  std::unique_ptr<FlatVariant>& slot = d->fvar[log2_words(V)][Q - 1][observe ? 1 : 0];
   if (slot) return slot.get();
   auto v = std::make_unique<FlatVariant>();
   const GateProgram& gp = d->gp();
@@ -292,6 +293,7 @@ FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q) {
   };
   FlatOptions o;
   o.warps = kFlatComputeThreads / 32 / Q;
+  o.observe = observe;
   v->fp = build_flat_program(gp, V, o);
   v->max_n = fit(v->fp.n_slots);
   if (v->max_n < top) {
@@ -412,11 +414,37 @@ uint32_t choose_tile_words(rrtl_design* d, uint32_t words) {
 // leaves most SMs idle.
 struct FlatShape {
   uint32_t V = 0, N = 1, Q = 1;
+  uint32_t words() const { return V * N * Q; }
 };
-FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w) {
+constexpr FlatShape kFlatShapes[] = {{4, 2, 2}, {4, 3, 1}, {4, 2, 1}, {4, 1, 1}, {2, 1, 1}, {1, 1, 1}};
+// The tile width a flat run reports: several tiles of the widest documented
+// width that divides its own.
+uint32_t flat_reported_words(uint32_t w) { return w == 16 ? 8 : w == 12 ? 4 : w; }
+
+// Clocks of one tile-cycle, from the statistics of the program built for row
+// width `base`.
+double flat_tile_cost(const FlatProgram& fp, uint32_t base, const FlatShape& x) {
+  const double vec4 = (double)fp.wavefronts * (base == 4 ? 1.0 : base == 2 ? 1.85 : 3.4);  // wavefronts of 4-word rows
+  const double work = vec4 * (x.V == 4 ? 1.2 * x.N * x.Q : x.V == 2 ? 0.58 : 0.36);
+  return fp.n_levels * 250.0 + fp.n_entries * 10.0 + work + 600.0;
+}
+
+// The widest rows that fit (0: none); packing leaves fewer live nets than the
+// fused program's slots.
+uint32_t flat_base(rrtl_design* d, bool observe) {
+  for (uint32_t V = 4; V >= 1; V /= 2)
+    if ((size_t)d->gp().n_slots * V * 4 <= flat_plane_bytes(1) / 4 * 5 && flat_variant(d, V, 1, observe)->max_n) return V;
+  return 0;
+}
+
+bool flat_fits(rrtl_design* d, const FlatShape& x, bool observe) {
+  return flat_variant(d, x.V, x.Q, observe)->max_n >= x.N * x.Q;
+}
+
+FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w, uint32_t tuned_w, bool observe) {
   FlatShape s;
   auto checked = [&](FlatShape x) {
-    if (x.V && flat_variant(d, x.V, x.Q)->max_n < x.N * x.Q) x.V = 0;
+    if (x.V && !flat_fits(d, x, observe)) x.V = 0;
     return x;
   };
   const char* env = getenv("RRTL_FLAT");
@@ -432,21 +460,14 @@ FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w) {
     s.N = explicit_w / s.V;
     return checked(s);
   }
-  // the widest rows that fit; packing leaves fewer live nets than the fused program's slots
-  uint32_t top = 0;
-  for (uint32_t V = 4; V >= 1 && !top; V /= 2)
-    if ((size_t)d->gp().n_slots * V * 4 <= flat_plane_bytes(1) / 4 * 5 && flat_variant(d, V, 1)->max_n) top = V;
+  const uint32_t top = flat_base(d, observe);
   if (!top) return s;
-  const FlatVariant* v = flat_variant(d, top, 1);
-  const FlatProgram& fp = v->fp;
-  const double vec4 = (double)fp.wavefronts * (top == 4 ? 1.0 : top == 2 ? 1.85 : 3.4);  // wavefronts of 4-word rows
-  const FlatShape shapes[] = {{4, 2, 2}, {4, 3, 1}, {4, 2, 1}, {4, 1, 1}, {2, 1, 1}, {1, 1, 1}};
+  const FlatVariant* v = flat_variant(d, top, 1, observe);
   double best = INFINITY;
-  for (const FlatShape& x : shapes) {
+  for (const FlatShape& x : kFlatShapes) {
     if (x.V > top || (x.V == 4 && x.N * x.Q > v->max_n)) continue;
-    const double work = vec4 * (x.V == 4 ? 1.2 * x.N * x.Q : x.V == 2 ? 0.58 : 0.36);
-    const double rounds = std::ceil(std::ceil((double)words / (x.V * x.N * x.Q)) / d->ctx->sm_count);
-    const double t = rounds * (fp.n_levels * 250.0 + fp.n_entries * 10.0 + work);
+    if (tuned_w && flat_reported_words(x.words()) != tuned_w) continue;
+    const double t = std::ceil(std::ceil((double)words / x.words()) / d->ctx->sm_count) * flat_tile_cost(v->fp, top, x);
     if (t < best) {
       best = t;
       s = x;
@@ -547,7 +568,62 @@ void build_forces(rrtl_batch* b, ForceTable& ft, uint32_t tile_words, const Gate
   ft.valid = true;
 }
 
+// The same for a flat program: forces of comb nets by (tile, writing warp,
+// level), of registers by tile.
+void build_flat_forces(rrtl_batch* b, const FlatVariant* fv, uint32_t N, uint32_t Q) {
+  FlatForceTable& ft = b->forces_flat;
+  const FlatProgram& fp = fv->fp;
+  const uint32_t V = fp.V, W = V * N * Q, shape = V * 100 + N * 10 + Q;
+  if (ft.shape == shape) return;
+  const GateProgram& gp = b->d->gp();
+  const uint32_t warps = fp.warps * Q, n_tiles = (b->words_pad + W - 1) / W;
+  struct F {
+    uint32_t key, level, off, mask, val;  // key: tile * warps + warp, or the tile of a register
+  };
+  std::vector<F> comb, regs;
+  for (size_t i = 0; i < b->faults.size(); ++i) {
+    const rrtl_fault& f = b->faults[i];
+    const uint32_t net = gp.signal_net[f.signal], gw = f.lane / 32, tile = gw / W, ww = gw % W, plane = ww / V;
+    if (fp.net_slot[net] < 0) continue;  // nothing reads the net within a cycle
+    const uint32_t off = plane * flat_plane_bytes(N * Q) + (uint32_t)fp.net_slot[net] * V * 4 + ww % V * 4;
+    const uint32_t bit = 1u << (f.lane % 32);
+    const F x{0, 0, off, bit, f.value ? bit : 0u};
+    if (gp.net_is_source[net]) {
+      regs.push_back(x);
+      regs.back().key = tile;
+    } else {
+      comb.push_back(x);
+      comb.back().key = tile * warps + plane / N * fp.warps + fp.net_warp[net];
+      comb.back().level = (uint32_t)fp.net_level[net];
+    }
+  }
+  // forces of one word together (a later fault on a lane wins), then lists with their offsets
+  auto finish = [&](std::vector<F>& v, uint32_t keys, DevBuf& d_off, DevBuf& d_forces) {
+    std::stable_sort(v.begin(), v.end(), [](const F& x, const F& y) {
+      return std::tie(x.key, x.level, x.off) < std::tie(y.key, y.level, y.off);
+    });
+    std::vector<uint32_t> off(keys + 1, 0);
+    std::vector<uint4> out;
+    for (size_t i = 0; i < v.size(); ++i) {
+      if (i && v[i].key == v[i - 1].key && v[i].level == v[i - 1].level && v[i].off == v[i - 1].off) {
+        out.back().y |= v[i].mask;
+        out.back().z = (out.back().z & ~v[i].mask) | v[i].val;
+        continue;
+      }
+      out.push_back(make_uint4(v[i].off, v[i].mask, v[i].val, v[i].level));
+      ++off[v[i].key + 1];
+    }
+    for (uint32_t k = 0; k < keys; ++k) off[k + 1] += off[k];
+    upload(d_off, off);
+    upload(d_forces, out);
+  };
+  finish(comb, n_tiles * warps, ft.d_off, ft.d_forces);
+  finish(regs, n_tiles, ft.d_off0, ft.d_forces0);
+  ft.shape = shape;
+}
+
 void invalidate_forces(rrtl_batch* b) {
+  b->forces_flat.shape = 0;
   b->forces_plain.valid = false;
   for (auto& f : b->forces_fused) f.valid = false;
 }
@@ -562,17 +638,20 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   rrtl_design* d = b->d;
   cudaStream_t st = d->ctx->stream;
   GatePrepared g;
-  if (want_flat && want_fused && run.cycles >= kFlatMinCycles && b->faults.empty() && d->gate_w_max) {
-    uint32_t ew = b->tile_words;
+  if (want_flat && want_fused && run.cycles >= kFlatMinCycles && d->gate_w_max) {
+    const bool observe = !b->faults.empty();
     auto tuned = d->tuned_w.find(lane_bucket(b->words));
-    if (!ew && tuned != d->tuned_w.end() && tuned->second != kTunedCompiled) ew = tuned->second;
-    const FlatShape fs = choose_flat(d, b->words, ew);
+    const uint32_t tw = tuned != d->tuned_w.end() && tuned->second != kTunedCompiled ? tuned->second : 0;
+    const FlatShape fs = choose_flat(d, b->words, b->tile_words, tw, observe);
+    const GateProgram& p = d->gp();
     bool ok = fs.V != 0;
     for (uint32_t i = 0; ok && i < run.n_record; ++i)
-      ok = run.record[i] < d->gp().signal_net.size() &&
-           flat_variant(d, fs.V, fs.Q)->fp.recordable[d->gp().signal_net[run.record[i]]];
+      ok = run.record[i] < p.signal_net.size() &&
+           flat_variant(d, fs.V, fs.Q, observe)->fp.recordable[p.signal_net[run.record[i]]];
+    for (uint32_t i = 0; ok && observe && i < run.n_stim; ++i)  // a forced register is no input
+      ok = run.stim[i].signal < p.signal_net.size() && d->mp.source.signals[run.stim[i].signal].kind != PSK::Reg;
     if (ok) {
-      g.flat = flat_variant(d, fs.V, fs.Q);
+      g.flat = flat_variant(d, fs.V, fs.Q, observe);
       g.flat_n = fs.N;
       g.flat_q = fs.Q;
     }
@@ -638,6 +717,13 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   R.force_off = ft.d_off.as<uint32_t>();
   R.forces = ft.d_forces.as<GateForceDev>();
   R.has_forces = ft.any ? 1u : 0u;
+  if (g.flat && R.has_forces) {
+    build_flat_forces(b, g.flat, g.flat_n, g.flat_q);
+    R.flat_off = b->forces_flat.d_off.as<uint32_t>();
+    R.flat_forces = b->forces_flat.d_forces.as<uint4>();
+    R.flat_off0 = b->forces_flat.d_off0.as<uint32_t>();
+    R.flat_forces0 = b->forces_flat.d_forces0.as<uint4>();
+  }
   R.final_settle = 1;
   R.nets = b->d_nets.as<uint32_t>();
   R.err = b->d_err.as<uint32_t>();
@@ -818,8 +904,7 @@ void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckT
     g.W = 0;
   } else if (g.flat && g.fused) {
     gate_flat_launch(d, g, st);
-    g.W = g.flat->fp.V * g.flat_n * g.flat_q;
-    if (g.W > 8) g.W = g.W == 16 ? 8 : 4;  // several tiles of the widest documented width that divides them
+    g.W = flat_reported_words(g.flat->fp.V * g.flat_n * g.flat_q);
   } else if (g.fused) {
     uint32_t grid = std::min<uint32_t>(g.R.n_tiles, d->ctx->sm_count * g.v->fused_ctas);
     if (F)
@@ -2377,7 +2462,7 @@ rrtl_status rrtl_design_autotune(rrtl_design* d, uint32_t lanes, uint32_t cycles
       rrtl_batch* b = nullptr;
       rrtl_status st = rrtl_batch_create(d, lanes, &b);
       if (st) fail(st, g_last_error);
-      b->tile_words = W;
+      d->tuned_w[lane_bucket(words)] = W;  // as batches will run it once tuned
       float t = INFINITY;
       try {
         for (int rep = 0; rep < 3; ++rep) {

@@ -83,6 +83,12 @@ struct ForceTable {
   DevBuf d_off, d_forces;
 };
 
+// The same for one shape of the flat kernel.
+struct FlatForceTable {
+  uint32_t shape = 0;  // V * 100 + N * 10 + Q it was built for, 0: none
+  DevBuf d_off, d_forces, d_off0, d_forces0;
+};
+
 // A gate-engine run made ready for a launch: program variant, device run
 // descriptor and the sizes of its outputs.
 struct GatePrepared {
@@ -224,7 +230,7 @@ struct rrtl_design {
   // gate engine: one program per fused tile width W (index log2 W), built on
   // demand; nets, levels and registers are the same in every variant
   std::unique_ptr<rrtl::GateVariant> gvar[4];
-  std::unique_ptr<rrtl::FlatVariant> fvar[3][2];  // flat programs by log2 V and warp sets - 1
+  std::unique_ptr<rrtl::FlatVariant> fvar[3][2][2];  // flat programs by log2 V, warp sets - 1, with a row for every signal
   uint32_t gate_base = 3;   // log2 W of the variant built at load time
   uint32_t gate_w_max = 0;  // widest W whose slots fit on chip, 0 if none
   std::map<uint32_t, uint32_t> tuned_w;  // measured best W by lane bucket (ceil log2 of 32-lane words);
@@ -257,6 +263,7 @@ struct rrtl_batch {
   uint32_t last_tile_words = 0;  // tile width of the last fused run, 0 after a plain run
   rrtl::DevBuf d_nets;
   std::vector<rrtl_fault> faults;
+  rrtl::FlatForceTable forces_flat;
   rrtl::ForceTable forces_plain, forces_fused[4];  // plain: 8-word tiles; fused: per log2 W
   // word engine state
   uint32_t lanes_pad = 0;

@@ -44,10 +44,15 @@ extern "C" int emu_flat_run(const char* json, size_t len, const char* top, uint3
     GateProgram gp = build_gate_program(mp, 8);
     FlatOptions opt;
     opt.pack = pack != 0;
+    opt.observe = pack == 2;  // 2: every signal keeps a row
     opt.fold_regs = fold != 0;
     opt.warps = warps;
     opt.max_slots = max_slots;
     FlatProgram fp = build_flat_program(gp, V, opt);
+    for (uint32_t s = 0; opt.observe && s < gp.n_signals; ++s) {
+      const uint32_t net = gp.signal_net[s];
+      if (!gp.net_is_source[net] && fp.net_slot[net] >= 0 && fp.net_level[net] < 0) throw Fail{"a row no cell writes"};
+    }
     if (stats) {
       const uint32_t s[] = {fp.n_two,   fp.n_three, fp.n_levels, fp.n_slots, fp.n_entries, (uint32_t)fp.wavefronts,
                             (uint32_t)fp.floor_wavefronts, (uint32_t)fp.commit.size()};

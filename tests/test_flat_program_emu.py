@@ -71,7 +71,7 @@ def netlist():
 
 
 @pytest.mark.parametrize("V,warps", [(4, 16), (4, 8), (2, 16), (1, 16)])
-@pytest.mark.parametrize("pack,fold", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("pack,fold", [(0, 0), (1, 0), (0, 1), (1, 1), (2, 1)])
 def test_netlist_equals_the_oracle(emu, netlist, V, warps, pack, fold):
     js, meta, od = netlist
     stim, rec = netlist_run_spec(meta)

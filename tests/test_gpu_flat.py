@@ -109,3 +109,29 @@ def test_registers_on_the_commit_list(engine, monkeypatch, shape):
     assert g.tile_words != 0
     ref = _ref(od, 1000, 60, 9, stim, rec, 3)
     assert np.array_equal(res["trace"], ref["trace"]) and np.array_equal(res["hash"], ref["hash"])
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_stuck_at_faults(wide, monkeypatch, shape):
+    """Many faults on few lanes (more than a 32-force window per warp), on
+    wires, registers, outputs, several on one lane, two on one net."""
+    from rrtl_gb300.workloads import Rng
+
+    cd, meta, od = wide
+    monkeypatch.setenv("RRTL_FLAT", shape)
+    rng = Rng(int(shape))
+    lanes, cycles = 540, 14
+    sites = meta.gate_names + meta.regs + meta.outputs
+    faults = [(l, sites[rng.below(len(sites))], rng.below(2)) for l in range(lanes) if l % 32 for _ in range(1 + 8 * (l < 64))]
+    faults += [(33, meta.regs[3], 1), (33, meta.regs[3], 0), (34, meta.gate_names[5], 0), (34, meta.gate_names[5], 1)]
+    stim, rec = netlist_run_spec(meta, uniform=True)
+    mode = sim.REC_TRACE | sim.REC_HASH | sim.REC_DETECT
+    g = sim.GpuBatchSimulator(cd, lanes=lanes)
+    g.set_faults(faults)
+    res = g.run(cycles, seed=3, stim=stim, record=rec, mode=mode)
+    assert g.tile_words == {12: 4, 16: 8}.get(SHAPES[shape], SHAPES[shape])
+    ref = _ref(od, lanes, cycles, 3, stim, rec, mode, faults=[(l, od.signal(s), v) for l, s, v in faults])
+    for k in ("trace", "hash", "detect"):
+        assert np.array_equal(res[k], ref[k]), k
+    for n in meta.regs:
+        assert np.array_equal(g.get_signal_bits(n), ref["sim"].get_bits(od.signal(n))), n
