@@ -22,7 +22,7 @@ constexpr uint32_t kFlatConst0 = 0xFFFFFFFEu, kFlatConst1 = 0xFFFFFFFFu;  // con
 // Shared memory of the CTA: all of an SM's, so that the distance of the
 // tile's N planes is a compile-time constant.
 constexpr uint32_t kFlatSmem = 227 * 1024;
-constexpr uint32_t kFlatHeader = 256;
+constexpr uint32_t kFlatHeader = 512;  // detection state, the queue's item and job
 #if defined(__CUDACC__)
 __host__ __device__
 #endif

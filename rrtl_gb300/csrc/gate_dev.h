@@ -151,6 +151,20 @@ struct GateItemDev {
   uint32_t ncyc, flags;
 };
 
+// One job of the flat queue kernel and its launch.
+struct FlatJobDev {
+  FlatProgDev P;
+  GateRunDev R;
+  uint32_t shape, pad;  // V * 100 + N * 10 + Q
+};
+
+struct FlatQueueDev {
+  const FlatJobDev* jobs;
+  const GateItemDev* items;
+  uint32_t n_items;
+  uint32_t* next;  // atomic item counter, zeroed before the launch
+};
+
 struct GateQueueDev {
   const GateJobDev* jobs;
   const GateItemDev* items;

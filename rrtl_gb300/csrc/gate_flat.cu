@@ -39,4 +39,45 @@ cudaError_t launch_gate_flat(uint32_t V, uint32_t N, uint32_t Q, const FlatProgD
   }
 }
 
+// Persistent queue kernel: CTAs take (job, tile) items, all cycles of the
+// job, from a device list (longest first) until it is empty. The job's
+// descriptor lies in the header of shared memory, behind the detection state.
+template <int V, int N, int Q>
+__device__ __forceinline__ void queue_tile(const FlatJobDev& J, const GateItemDev& item, uint8_t* smem) {
+  if (J.R.has_forces) flat_tile<V, N, Q, true>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
+  else flat_tile<V, N, Q, false>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
+}
+
+__global__ void __launch_bounds__(kFlatThreads, 1) gate_flat_queue_kernel(FlatQueueDev L) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  uint32_t& s_item = *reinterpret_cast<uint32_t*>(smem + 128);
+  FlatJobDev& J = *reinterpret_cast<FlatJobDev*>(smem + 136);
+  static_assert(136 + sizeof(FlatJobDev) <= kFlatHeader, "the job descriptor overflows the header");
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(L.next, 1u);
+    __syncthreads();
+    const uint32_t it = s_item;
+    if (it >= L.n_items) break;
+    const GateItemDev item = L.items[it];
+    for (uint32_t i = threadIdx.x; i < sizeof(FlatJobDev) / 4; i += blockDim.x)
+      reinterpret_cast<uint32_t*>(&J)[i] = reinterpret_cast<const uint32_t*>(L.jobs + item.job)[i];
+    __syncthreads();  // also orders the s_item read before its next write
+    switch (J.shape) {
+      case 422: queue_tile<4, 2, 2>(J, item, smem); break;
+      case 421: queue_tile<4, 2, 1>(J, item, smem); break;
+      case 411: queue_tile<4, 1, 1>(J, item, smem); break;
+      case 211: queue_tile<2, 1, 1>(J, item, smem); break;
+      case 111: queue_tile<1, 1, 1>(J, item, smem); break;
+      default: break;
+    }
+  }
+}
+
+cudaError_t launch_gate_flat_queue(const FlatQueueDev& L, uint32_t grid, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(gate_flat_queue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlatSmem);
+  if (e != cudaSuccess) return e;
+  gate_flat_queue_kernel<<<grid, kFlatThreads, kFlatSmem, st>>>(L);
+  return cudaGetLastError();
+}
+
 }  // namespace rrtl

@@ -23,6 +23,7 @@ int gate_fused_ctas_per_sm(const GateProgDev& P, size_t smem);
 cudaError_t launch_gate_fused(const GateProgDev& P, const GateRunDev& R, uint32_t grid, size_t smem, cudaStream_t st);
 cudaError_t launch_gate_flat(uint32_t V, uint32_t N, uint32_t Q, const FlatProgDev& P, const GateRunDev& R, uint32_t grid,
                              cudaStream_t st);
+cudaError_t launch_gate_flat_queue(const FlatQueueDev& L, uint32_t grid, cudaStream_t st);
 cudaError_t launch_gate_plain(const GateProgDev& P, const GateRunDev& R, uint64_t c, int phase, cudaStream_t st);
 cudaError_t launch_word(const WordProgDev& P, const WordRunDev& R, bool smem_slots, cudaStream_t st);
 cudaError_t word_prepare(size_t smem);
@@ -412,10 +413,6 @@ uint32_t choose_tile_words(rrtl_design* d, uint32_t words) {
 // of two: 100.1k as one set). So a tile costs about 250 clocks a level, 10 an
 // entry and 1.2 a wavefront, and wide tiles pay until the last round of tiles
 // leaves most SMs idle.
-struct FlatShape {
-  uint32_t V = 0, N = 1, Q = 1;
-  uint32_t words() const { return V * N * Q; }
-};
 constexpr FlatShape kFlatShapes[] = {{4, 2, 2}, {4, 3, 1}, {4, 2, 1}, {4, 1, 1}, {2, 1, 1}, {1, 1, 1}};
 // The tile width a flat run reports: several tiles of the widest documented
 // width that divides its own.
@@ -628,33 +625,47 @@ void invalidate_forces(rrtl_batch* b) {
   for (auto& f : b->forces_fused) f.valid = false;
 }
 
+// Whether the flat kernel can take a run: long enough, every recorded net in
+// a row at the end of a cycle, no stimulus on a register that may be forced.
+bool flat_takes(rrtl_batch* b, const rrtl_run& run) {
+  rrtl_design* d = b->d;
+  const char* env = getenv("RRTL_FLAT");
+  if ((env && env[0] == '0') || run.cycles < kFlatMinCycles || !d->gate_w_max) return false;
+  const bool observe = !b->faults.empty();
+  const uint32_t base = flat_base(d, observe);
+  if (!base) return false;
+  const GateProgram& p = d->gp();
+  const FlatProgram& fp = flat_variant(d, base, 1, observe)->fp;
+  for (uint32_t i = 0; i < run.n_record; ++i)
+    if (run.record[i] >= p.signal_net.size() || !fp.recordable[p.signal_net[run.record[i]]]) return false;
+  for (uint32_t i = 0; observe && i < run.n_stim; ++i)
+    if (run.stim[i].signal >= p.signal_net.size() || d->mp.source.signals[run.stim[i].signal].kind == PSK::Reg) return false;
+  return true;
+}
+
+uint32_t tuned_words(rrtl_design* d, uint32_t words) {
+  auto t = d->tuned_w.find(lane_bucket(words));
+  return t != d->tuned_w.end() && t->second != kTunedCompiled ? t->second : 0;
+}
+
+FlatShape flat_shape_for(rrtl_batch* b, const rrtl_run& run) {
+  if (!flat_takes(b, run)) return FlatShape{};
+  return choose_flat(b->d, b->words, b->tile_words, tuned_words(b->d, b->words), !b->faults.empty());
+}
+
 // ---- gate engine run
 // Validate a run, pick the program variant and upload its stimulus and record
 // tables; stages host input traces and zeroes hash/detect outputs on the
 // context stream. `want_fused` asks for the fused path (it falls back to the
 // plain path when a recorded net does not stay on chip to the end of a cycle).
 GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool want_fused,
-                          const CheckTables* chk, bool want_flat) {
+                          const CheckTables* chk, FlatShape flat) {
   rrtl_design* d = b->d;
   cudaStream_t st = d->ctx->stream;
   GatePrepared g;
-  if (want_flat && want_fused && run.cycles >= kFlatMinCycles && d->gate_w_max) {
-    const bool observe = !b->faults.empty();
-    auto tuned = d->tuned_w.find(lane_bucket(b->words));
-    const uint32_t tw = tuned != d->tuned_w.end() && tuned->second != kTunedCompiled ? tuned->second : 0;
-    const FlatShape fs = choose_flat(d, b->words, b->tile_words, tw, observe);
-    const GateProgram& p = d->gp();
-    bool ok = fs.V != 0;
-    for (uint32_t i = 0; ok && i < run.n_record; ++i)
-      ok = run.record[i] < p.signal_net.size() &&
-           flat_variant(d, fs.V, fs.Q, observe)->fp.recordable[p.signal_net[run.record[i]]];
-    for (uint32_t i = 0; ok && observe && i < run.n_stim; ++i)  // a forced register is no input
-      ok = run.stim[i].signal < p.signal_net.size() && d->mp.source.signals[run.stim[i].signal].kind != PSK::Reg;
-    if (ok) {
-      g.flat = flat_variant(d, fs.V, fs.Q, observe);
-      g.flat_n = fs.N;
-      g.flat_q = fs.Q;
-    }
+  if (flat.V) {
+    g.flat = flat_variant(d, flat.V, flat.Q, !b->faults.empty());
+    g.shape = flat;
   }
   // (the fused kernel only closes a flat run: the variant built at load time does)
   const uint32_t W = !want_fused ? 0
@@ -718,7 +729,7 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   R.forces = ft.d_forces.as<GateForceDev>();
   R.has_forces = ft.any ? 1u : 0u;
   if (g.flat && R.has_forces) {
-    build_flat_forces(b, g.flat, g.flat_n, g.flat_q);
+    build_flat_forces(b, g.flat, flat.N, flat.Q);
     R.flat_off = b->forces_flat.d_off.as<uint32_t>();
     R.flat_forces = b->forces_flat.d_forces.as<uint4>();
     R.flat_off0 = b->forces_flat.d_off0.as<uint32_t>();
@@ -781,20 +792,29 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   return g;
 }
 
-// A flat run: the cycles on the flat kernel, then the closing settle, which
-// writes every signal back, on the fused kernel.
-void gate_flat_launch(rrtl_design* d, const GatePrepared& g, cudaStream_t st) {
-  const uint32_t V = g.flat->fp.V, W = V * g.flat_n * g.flat_q;
+// Descriptors of a flat run's cycles, over the flat shape's tiles, and of its
+// closing settle, over the fused variant's.
+GateRunDev flat_run_desc(const GatePrepared& g) {
   GateRunDev R = g.R;
-  R.n_tiles = (g.R.words_pad + W - 1) / W;
-  cuda_check(launch_gate_flat(V, g.flat_n, g.flat_q, g.flat->dev, R, std::min(R.n_tiles, d->ctx->sm_count), st),
-             "gate_flat_kernel");
+  R.n_tiles = (g.R.words_pad + g.shape.words() - 1) / g.shape.words();
+  return R;
+}
+GateRunDev closing_desc(const GatePrepared& g) {
   GateRunDev C = g.R;
   C.cycles = 0;
   C.n_stim = 0;
   C.n_rec = 0;
   C.mode = 0;
   C.n_tiles = g.R.words_pad / g.W;
+  return C;
+}
+
+// A flat run: the cycles on the flat kernel, then the closing settle, which
+// writes every signal back, on the fused kernel.
+void gate_flat_launch(rrtl_design* d, const GatePrepared& g, cudaStream_t st) {
+  const GateRunDev R = flat_run_desc(g), C = closing_desc(g);
+  cuda_check(launch_gate_flat(g.shape.V, g.shape.N, g.shape.Q, g.flat->dev, R, std::min(R.n_tiles, d->ctx->sm_count), st),
+             "gate_flat_kernel");
   const uint32_t grid = std::min<uint32_t>(C.n_tiles, d->ctx->sm_count * g.v->fused_ctas);
   cuda_check(launch_gate_fused(g.v->gdev, C, grid, g.v->fused_smem, st), "gate_fused_kernel");
 }
@@ -892,11 +912,13 @@ void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckT
   cudaStream_t st = d->ctx->stream;
   const bool compiled = b->path == RRTL_PATH_FUSED && b->faults.empty() &&
                         (force_compiled || (b->tile_words == 0 && gate_jit_preferred(d, b->words)));
-  GatePrepared g = gate_prepare(b, run, device_ptrs, b->path == RRTL_PATH_FUSED, chk, !compiled);
+  const FlatShape fs = b->path == RRTL_PATH_FUSED && !compiled ? flat_shape_for(b, run) : FlatShape{};
+  GatePrepared g = gate_prepare(b, run, device_ptrs, b->path == RRTL_PATH_FUSED, chk, fs);
   // the compiled gate kernel: automatic tile width, no stuck-at forces; built before the timed region
   const JitKernel* J = compiled && !g.R.has_forces ? gate_jit_for_run(d, g.tables) : nullptr;
   // the fused kernel compiled for the design's truth-table classes, also built before the timed region
-  const JitKernel* F = !J && g.fused && !g.flat ? fused_jit_for(d, g.v) : nullptr;
+  // (not for a settle alone, which runs the same code in both)
+  const JitKernel* F = !J && g.fused && !g.flat && run.cycles ? fused_jit_for(d, g.v) : nullptr;
   Timer tm(b);
   if (J) {
     g.R.cycle_base = 0;
@@ -904,7 +926,7 @@ void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckT
     g.W = 0;
   } else if (g.flat && g.fused) {
     gate_flat_launch(d, g, st);
-    g.W = flat_reported_words(g.flat->fp.V * g.flat_n * g.flat_q);
+    g.W = flat_reported_words(g.shape.words());
   } else if (g.fused) {
     uint32_t grid = std::min<uint32_t>(g.R.n_tiles, d->ctx->sm_count * g.v->fused_ctas);
     if (F)
@@ -1237,24 +1259,106 @@ uint64_t queue_submit(rrtl_ctx* c, const rrtl_job& job) {
   return Q.jobs.back().id;
 }
 
+// Flat shapes of the queued jobs that the flat kernel takes (V = 0: the
+// fused kernel's queue). Each job starts with the shape of least total SM
+// time; while the longest item is longer than an even share of all items, its
+// job moves to the shape that lowers the launch's bound (the larger of the
+// two), so a long job on few lanes is split over narrow tiles and the others
+// keep the cheaper wide ones.
+std::vector<FlatShape> queue_shapes(rrtl_ctx* c, const std::vector<QueueJob*>& jobs) {
+  struct Choice {
+    FlatShape s;
+    double len, total;  // clocks of one item, of all of the job's items
+  };
+  std::vector<std::vector<Choice>> opts(jobs.size());
+  std::vector<size_t> at(jobs.size(), 0);
+  double sum = 0;
+  for (size_t i = 0; i < jobs.size(); ++i) {
+    rrtl_batch* b = jobs[i]->batch;
+    if (!flat_takes(b, jobs[i]->run)) continue;
+    const bool observe = !b->faults.empty();
+    const uint32_t base = flat_base(b->d, observe), tw = tuned_words(b->d, b->words);
+    const FlatVariant* v = flat_variant(b->d, base, 1, observe);
+    auto add = [&](FlatShape x) {
+      const double len = (double)jobs[i]->run.cycles * flat_tile_cost(v->fp, base, x);
+      opts[i].push_back(Choice{x, len, len * std::ceil((double)b->words / x.words())});
+    };
+    for (const FlatShape& x : kFlatShapes) {
+      if (x.words() == 12) continue;  // not built into the queue kernel
+      if (x.V > base || (x.V == 4 && x.N * x.Q > v->max_n)) continue;
+      if (b->tile_words ? x.words() != b->tile_words : tw && flat_reported_words(x.words()) != tw) continue;
+      add(x);
+    }
+    for (size_t k = 1; k < opts[i].size(); ++k)
+      if (opts[i][k].total < opts[i][at[i]].total) at[i] = k;
+    if (!opts[i].empty()) sum += opts[i][at[i]].total;
+  }
+  const double sms = c->sm_count;
+  for (size_t moves = 0; moves < jobs.size() * 6; ++moves) {
+    size_t big = jobs.size();
+    double len = 0, second = 0;
+    for (size_t i = 0; i < jobs.size(); ++i) {
+      if (opts[i].empty()) continue;
+      const double l = opts[i][at[i]].len;
+      if (l > len) {
+        second = len;
+        len = l;
+        big = i;
+      } else {
+        second = std::max(second, l);
+      }
+    }
+    if (big == jobs.size() || len <= sum / sms) break;
+    size_t best = at[big];
+    double bound = len;
+    for (size_t k = 0; k < opts[big].size(); ++k) {
+      const Choice& x = opts[big][k];
+      const double t = std::max(std::max(x.len, second), (sum - opts[big][at[big]].total + x.total) / sms);
+      if (x.len < len && (t < bound || (t == bound && x.len < opts[big][best].len))) {
+        bound = t;
+        best = k;
+      }
+    }
+    if (best == at[big]) break;
+    sum += opts[big][best].total - opts[big][at[big]].total;
+    at[big] = best;
+  }
+  std::vector<FlatShape> out(jobs.size());
+  for (size_t i = 0; i < jobs.size(); ++i)
+    if (!opts[i].empty()) {
+      const FlatShape x = opts[i][at[i]].s;
+      if (flat_fits(jobs[i]->batch->d, x, !jobs[i]->batch->faults.empty())) out[i] = x;
+    }
+  return out;
+}
+
 // One persistent launch over every queued job: each job's tiles become items
-// (all cycles of one tile), listed longest first; jobs whose recorded nets
-// leave the chip, or whose shared memory exceeds what the queue kernel can
-// take, run on their own kernels first on the same stream.
+// (all cycles of one tile), listed longest first. Jobs the flat kernel takes
+// run there and leave their closing settle to the fused queue kernel behind
+// it, which also runs the other jobs; jobs whose recorded nets leave the chip,
+// or whose shared memory exceeds what the queue kernel can take, run on their
+// own kernels first on the same stream.
 void queue_launch(rrtl_ctx* c) {
   JobQueue& Q = queue_of(c);
   cudaStream_t st = c->stream;
   const size_t qmax = c->max_smem - gate_queue_static_smem();
   std::vector<GateJobDev> jobs;
-  std::vector<std::pair<double, GateItemDev>> items;
+  std::vector<FlatJobDev> flat_jobs;
+  using Item = std::pair<double, GateItemDev>;
+  std::vector<Item> items, flat_items;
   size_t smem = 0;
   const uint32_t launch = ++Q.launches;
+  std::vector<QueueJob*> todo;
+  for (QueueJob& j : Q.jobs)
+    if (j.status == RRTL_JOB_QUEUED) todo.push_back(&j);
+  std::vector<FlatShape> shapes = queue_shapes(c, todo);
   cuda_check(cudaEventRecord(Q.ev0, st), "event");
-  for (QueueJob& j : Q.jobs) {
-    if (j.status != RRTL_JOB_QUEUED) continue;
+  for (size_t i = 0; i < todo.size(); ++i) {
+    QueueJob& j = *todo[i];
     rrtl_batch* b = j.batch;
     b->path = RRTL_PATH_FUSED;
-    j.prep = gate_prepare(b, j.run, false, true);
+    if (shapes[i].V && gate_variant(b->d, b->d->gate_w_max)->fused_smem > qmax) shapes[i].V = 0;
+    j.prep = gate_prepare(b, j.run, false, true, nullptr, shapes[i]);
     j.status = RRTL_JOB_RUNNING;
     j.launch = launch;
     const GatePrepared& g = j.prep;
@@ -1269,33 +1373,51 @@ void queue_launch(rrtl_ctx* c) {
       continue;
     }
     const uint32_t ji = (uint32_t)jobs.size();
-    jobs.push_back(GateJobDev{g.v->gdev, g.R});
     smem = std::max(smem, g.v->fused_smem);
-    const double cost = (double)(j.run.cycles + 1) * g.v->tile_cycle_cost;
-    for (uint32_t t = 0; t < g.R.n_tiles; ++t)
-      items.push_back({cost, GateItemDev{ji, t, 0ull, (uint32_t)j.run.cycles, 1u}});
-    b->last_tile_words = g.W;
+    if (g.flat) {
+      const GateRunDev R = flat_run_desc(g);
+      const double cost = (double)j.run.cycles * flat_tile_cost(g.flat->fp, g.shape.V, g.shape);
+      for (uint32_t t = 0; t < R.n_tiles; ++t)
+        flat_items.push_back({cost, GateItemDev{(uint32_t)flat_jobs.size(), t, 0ull, (uint32_t)j.run.cycles, 0u}});
+      flat_jobs.push_back(FlatJobDev{g.flat->dev, R, g.shape.V * 100 + g.shape.N * 10 + g.shape.Q, 0u});
+      jobs.push_back(GateJobDev{g.v->gdev, closing_desc(g)});
+      b->last_tile_words = flat_reported_words(g.shape.words());
+    } else {
+      jobs.push_back(GateJobDev{g.v->gdev, g.R});
+      b->last_tile_words = g.W;
+    }
+    const uint64_t cycles = jobs.back().R.cycles;
+    const double cost = (double)(cycles + 1) * g.v->tile_cycle_cost;
+    for (uint32_t t = 0; t < jobs.back().R.n_tiles; ++t)
+      items.push_back({cost, GateItemDev{ji, t, 0ull, (uint32_t)cycles, 1u}});
   }
-  std::stable_sort(items.begin(), items.end(),
-                   [](const std::pair<double, GateItemDev>& x, const std::pair<double, GateItemDev>& y) {
-                     return x.first > y.first;
-                   });
-  Q.last_items = (uint32_t)items.size();
-  if (!items.empty()) {
+  Q.last_items = (uint32_t)(items.size() + flat_items.size());
+  auto stage = [&](std::vector<Item>& v, DevBuf& d) {
+    std::stable_sort(v.begin(), v.end(), [](const Item& x, const Item& y) { return x.first > y.first; });
     std::vector<GateItemDev> flat;
-    flat.reserve(items.size());
-    for (auto& it : items) flat.push_back(it.second);
+    flat.reserve(v.size());
+    for (auto& it : v) flat.push_back(it.second);
+    upload(d, flat);
+  };
+  if (!items.empty()) {
+    stage(items, Q.d_items);
     upload(Q.d_jobs, jobs);
-    upload(Q.d_items, flat);
     Q.d_next.reserve(16);
-    cuda_check(cudaMemsetAsync(Q.d_next.p, 0, 8, st), "memset queue");
+    cuda_check(cudaMemsetAsync(Q.d_next.p, 0, 16, st), "memset queue");
+    if (!flat_items.empty()) {
+      stage(flat_items, Q.d_flat_items);
+      upload(Q.d_flat_jobs, flat_jobs);
+      FlatQueueDev L{Q.d_flat_jobs.as<FlatJobDev>(), Q.d_flat_items.as<GateItemDev>(), (uint32_t)flat_items.size(),
+                     Q.d_next.as<uint32_t>() + 2};
+      cuda_check(launch_gate_flat_queue(L, std::min<uint32_t>(L.n_items, c->sm_count), st), "gate_flat_queue_kernel");
+    }
     if (!Q.smem_set) {
       // the limit is per kernel: allow every job this queue can take
       cuda_check(gate_queue_prepare(qmax), "gate_queue_prepare");
       Q.smem_set = qmax;
     }
-    GateQueueDev QD{Q.d_jobs.as<GateJobDev>(), Q.d_items.as<GateItemDev>(), (uint32_t)flat.size(), Q.d_next.as<uint32_t>()};
-    const uint32_t grid = std::min<uint32_t>((uint32_t)flat.size(), c->sm_count);
+    GateQueueDev QD{Q.d_jobs.as<GateJobDev>(), Q.d_items.as<GateItemDev>(), (uint32_t)items.size(), Q.d_next.as<uint32_t>()};
+    const uint32_t grid = std::min<uint32_t>((uint32_t)items.size(), c->sm_count);
     cuda_check(launch_gate_queue(QD, grid, smem, st), "gate_queue_kernel");
   }
   cuda_check(cudaEventRecord(Q.ev1, st), "event");

@@ -76,6 +76,13 @@ struct FlatVariant {
   DevBuf d_stream, d_warps, d_src_net, d_src_slot, d_commit;
 };
 
+// A shape of the flat kernel: row width V (0: none), vectors per warp set N,
+// warp sets Q.
+struct FlatShape {
+  uint32_t V = 0, N = 1, Q = 1;
+  uint32_t words() const { return V * N * Q; }
+};
+
 // Per-tile, per-stage force table of a batch for one tile width.
 struct ForceTable {
   bool valid = false;
@@ -99,7 +106,7 @@ struct GatePrepared {
   uint32_t W = 0;
   // the flat kernel runs the cycles and the fused kernel the closing settle
   FlatVariant* flat = nullptr;
-  uint32_t flat_n = 0, flat_q = 0;  // vectors per warp set, warp sets
+  FlatShape shape;
   size_t trace_out_bytes = 0, hash_bytes = 0, det_bytes = 0;
   bool want_trace = false, want_hash = false, want_det = false;
 };
@@ -132,7 +139,7 @@ struct JobQueue {
   uint32_t launches = 0;
   std::vector<QueueJob> jobs;                 // queued or running
   std::unordered_map<uint64_t, uint32_t> finished;  // id -> RRTL_JOB_DONE / RRTL_JOB_FAILED
-  DevBuf d_jobs, d_items, d_next;
+  DevBuf d_jobs, d_items, d_next, d_flat_jobs, d_flat_items;
   size_t smem_set = 0;                        // dynamic shared memory the queue kernel is prepared for
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;   // around the last launch
   float last_ms = 0.f;
@@ -150,7 +157,7 @@ struct CheckTables {
 
 // Runtime internals shared by the C ABI and the serving loop.
 GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool want_fused,
-                          const CheckTables* chk = nullptr, bool want_flat = false);
+                          const CheckTables* chk = nullptr, FlatShape flat = FlatShape{});
 void gate_copy_out(rrtl_batch* b, const GatePrepared& g, const rrtl_run& run);
 void gate_plain_launches(const GatePrepared& g, uint64_t cycles, cudaStream_t st, bool graph);
 WordPrepared word_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool start_settle,

@@ -135,3 +135,40 @@ def test_stuck_at_faults(wide, monkeypatch, shape):
         assert np.array_equal(res[k], ref[k]), k
     for n in meta.regs:
         assert np.array_equal(g.get_signal_bits(n), ref["sim"].get_bits(od.signal(n))), n
+
+
+def test_queue_of_flat_and_fused_jobs(wide, monkeypatch):
+    """One launch of jobs of every size (a long one on one lane, wide ones,
+    one too short for the flat kernel, fault jobs, an explicit tile width)
+    equals the same runs alone on the fused kernel."""
+    from rrtl_gb300.workloads import job_faults
+
+    cd, meta, od = wide
+    jobs = [(1, 400, 0, 0), (3000, 20, 0, 0), (77, 2, 0, 0), (640, 30, 1, 0), (2048, 9, 1, 0), (33, 50, 0, 2), (900, 8, 0, 8)]
+    out = {}
+    for flat in ("", "0"):
+        monkeypatch.setenv("RRTL_FLAT", flat)
+        ctx = sim.default_context()
+        queued, keep = [], []
+        for i, (lanes, cycles, fault, words) in enumerate(jobs):
+            g = sim.GpuBatchSimulator(cd, lanes=lanes)
+            g.set_tile_words(words)
+            if fault:
+                g.set_faults(job_faults(meta, lanes, i))
+            stim, rec = netlist_run_spec(meta, uniform=bool(fault))
+            mode = sim.REC_HASH | sim.REC_TRACE | (sim.REC_DETECT if fault else 0)
+            keep.append(g)
+            if flat == "":
+                queued.append(ctx.submit(g, cycles, seed=i, stim=stim, record=rec, mode=mode))
+            else:
+                queued.append(g.run(cycles, seed=i, stim=stim, record=rec, mode=mode))
+        if flat == "":
+            ctx.launch()
+            ctx.wait()
+            assert [j.status for j in queued] == [sim.JOB_DONE] * len(jobs)
+            queued = [j.outputs for j in queued]
+        out[flat] = [(r, g.get_signals_bits(meta.regs + meta.gate_names[::97])) for r, g in zip(queued, keep)]
+    for (a, sa), (b, sb) in zip(out[""], out["0"]):
+        for k in ("trace", "hash", "detect"):
+            assert (a[k] is None and b[k] is None) or np.array_equal(a[k], b[k]), k
+        assert np.array_equal(sa, sb)
