@@ -6,8 +6,8 @@
 // docs/rrtl-optimizations.md:1725-1734). Here a gate program (gateprog.h)
 // with its run's stimulus and record tables is emitted as straight-line CUDA
 // C++: one thread per 32-lane word for all cycles, every net a register, one
-// LOP3 per cell in level order, the register commit and the record stage
-// unrolled with the run's nets as constants. It serves runs without stuck-at
+// LOP3 per cell in level order and the register commit unrolled; the random
+// or traced stimulus and the record stage run on other warps of its block. It serves runs without stuck-at
 // forces on designs of up to kGateJitMaxCells cells; others run the fused
 // kernel.
 #pragma once
@@ -24,7 +24,6 @@
 namespace rrtl {
 
 constexpr size_t kGateJitMaxCells = 8192;
-constexpr uint32_t kGateJitThreads = 64;
 
 // A gate run's stimulus table (net, kind, param), record table (net) and
 // record mode: what the compiled kernel bakes in.
@@ -35,10 +34,13 @@ struct GateRunTables {
   std::string key() const;
 };
 
-std::string gate_jit_source(const GateProgram& gp, const GateRunTables& run);
+// service: the most service warps of a block (stimulus and record); 0: the
+// warp that evaluates the cells does both.
+std::string gate_jit_source(const GateProgram& gp, const GateRunTables& run, uint32_t service = 7);
+uint32_t gate_jit_threads(const GateRunTables& run, uint32_t service);  // of its blocks
 
 // Emit, compile and load; never throws (failures leave ok = false).
-void gate_jit_build(const GateProgram& gp, const GateRunTables& run, int device, JitKernel* J);
+void gate_jit_build(const GateProgram& gp, const GateRunTables& run, uint32_t service, int device, JitKernel* J);
 
 cudaError_t launch_gate_jit(const JitKernel& J, const GateRunDev& R, cudaStream_t st);
 

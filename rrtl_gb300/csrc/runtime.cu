@@ -877,13 +877,24 @@ const JitKernel* jit_cache_get(std::mutex& mu, std::map<std::string, std::unique
   return J->ok ? J : nullptr;
 }
 
-const JitKernel* gate_jit_for_run(rrtl_design* d, const GateRunTables& t) {
+const JitKernel* gate_jit_for_run(rrtl_design* d, const GateRunTables& t, uint32_t words) {
   const char* env = getenv("RRTL_GATE_JIT");
   if ((env && env[0] == '0') || d->gp().n_real_cells > kGateJitMaxCells || t.stim.size() > kJitRunTableMax ||
       t.rec.size() > kJitRunTableMax)
     return nullptr;
-  return jit_cache_get(d->wjit_mu, d->gjit_runs, t.key(),
-                       [&](JitKernel* J) { gate_jit_build(d->gp(), t, d->ctx->device, J); });
+  // Seven service warps with a block an SM; three with two blocks, which then
+  // still share the SM at 255 registers a thread, for runs that hash many
+  // records; none beyond, where the SMs have warps enough (us per cycle, none
+  // / three / seven, 155,648 lanes: crc32 hashed 1.30 / 0.91 / 0.65, without
+  // records 0.33 / 0.26 / 0.23; 262,144 lanes: crc32 hashed 1.30 / 1.06 /
+  // 1.28, 150 gates with 8 hashed outputs 0.54 / 0.63 / 0.56, without records
+  // 0.30 / 0.35 / 0.36; 524,288 lanes: crc32 hashed 1.28 / - / 2.54).
+  const uint32_t blocks = (words + 31) / 32, sms = d->ctx->sm_count;
+  uint32_t service = blocks <= sms ? 7 : blocks <= 2 * sms && (t.mode & RRTL_REC_HASH) && t.rec.size() >= 16 ? 3 : 0;
+  const char* senv = getenv("RRTL_GATE_JIT_SERVICE");  // A/B switch
+  if (senv && senv[0]) service = (uint32_t)(senv[0] - '0');
+  return jit_cache_get(d->wjit_mu, d->gjit_runs, t.key() + "|" + std::to_string(service),
+                       [&](JitKernel* J) { gate_jit_build(d->gp(), t, service, d->ctx->device, J); });
 }
 
 // The fused kernel compiled for this design's truth-table classes at tile
@@ -915,7 +926,7 @@ void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckT
   const FlatShape fs = b->path == RRTL_PATH_FUSED && !compiled ? flat_shape_for(b, run) : FlatShape{};
   GatePrepared g = gate_prepare(b, run, device_ptrs, b->path == RRTL_PATH_FUSED, chk, fs);
   // the compiled gate kernel: automatic tile width, no stuck-at forces; built before the timed region
-  const JitKernel* J = compiled && !g.R.has_forces ? gate_jit_for_run(d, g.tables) : nullptr;
+  const JitKernel* J = compiled && !g.R.has_forces ? gate_jit_for_run(d, g.tables, b->words) : nullptr;
   // the fused kernel compiled for the design's truth-table classes, also built before the timed region
   // (not for a settle alone, which runs the same code in both)
   const JitKernel* F = !J && g.fused && !g.flat && run.cycles ? fused_jit_for(d, g.v) : nullptr;

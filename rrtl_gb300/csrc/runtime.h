@@ -173,7 +173,7 @@ void set_last_error(const std::string& msg);
 WordRunDev word_chunk_desc(const WordPrepared& g, uint64_t c0, uint64_t n, bool last);
 // The compiled gate kernel for this run's tables (built on first use and
 // kept per design), or nullptr when the design or run does not qualify.
-const JitKernel* gate_jit_for_run(rrtl_design* d, const GateRunTables& t);
+const JitKernel* gate_jit_for_run(rrtl_design* d, const GateRunTables& t, uint32_t words);
 // Whether a fused-path run of `words` 32-lane words should use the compiled
 // gate kernel: the autotuner's choice for the lane bucket, else designs whose
 // live nets fit in registers.

@@ -24,10 +24,14 @@ RRTL_HD uint64_t smix64(uint64_t z) {
   return z ^ (z >> 31);
 }
 
-// 32 stimulus bits for (seed, stream, cycle, idx).
+// 32 stimulus bits for (seed, stream, cycle, idx), by way of a key of the
+// stream that holds for a whole run.
+RRTL_HD uint64_t stim_stream_key(uint64_t seed, uint64_t stream) { return smix64(seed ^ (stream * 0xD6E8FEB86659FD93ull)); }
+RRTL_HD uint32_t stim_key_word(uint64_t key, uint64_t cycle, uint64_t idx) {
+  return (uint32_t)smix64(key ^ (cycle * 0xA0761D6478BD642Full) ^ (idx * 0xE7037ED1A0B428DBull));
+}
 RRTL_HD uint32_t stim_word(uint64_t seed, uint64_t stream, uint64_t cycle, uint64_t idx) {
-  uint64_t k = smix64(seed ^ (stream * 0xD6E8FEB86659FD93ull));
-  return (uint32_t)smix64(k ^ (cycle * 0xA0761D6478BD642Full) ^ (idx * 0xE7037ED1A0B428DBull));
+  return stim_key_word(stim_stream_key(seed, stream), cycle, idx);
 }
 
 // Value of limb `limb` of a RANDOM input of `width` bits on global lane

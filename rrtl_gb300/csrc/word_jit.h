@@ -63,6 +63,7 @@ struct JitKernel {
   std::string error;     // why there is no compiled kernel (empty when ok)
   double compile_ms = 0; // emit + NVRTC + load
   size_t source_bytes = 0;
+  uint32_t threads = 0;          // block size of a compiled gate kernel
   size_t static_smem = 0;        // the kernel's static shared memory (stimulus/record tables)
   bool reg_signals = false;      // signal words live in registers (no signal staging)
   bool split = false;            // two warps per 32 lanes (word_jit_run_split)

@@ -88,3 +88,27 @@ def test_faults_and_explicit_widths_use_the_fused_kernel(engine):
     g2.set_tile_words(4)
     g2.run(10, stim=stim, record=rec, mode=sim.REC_HASH)
     assert g2.tile_words == 4
+
+
+@pytest.mark.parametrize("service", ["0", "1", "3", "7"])
+@pytest.mark.parametrize("lanes,cycles", [(1, 1), (70, 2), (1000, 31), (1056, 32), (2049, 33), (5000, 100)])
+def test_service_warps_equal_the_oracle(engine, monkeypatch, service, lanes, cycles):
+    """Stimulus and records on any number of service warps, over cycle counts
+    around the hash bursts (32 cycles) and lanes around the blocks (1,024),
+    with drawn, uniform, traced, constant and held inputs."""
+    monkeypatch.setenv("RRTL_GATE_JIT_SERVICE", service)
+    d, meta = gate_netlist(n_gates=170, n_ff=20, n_pi=9, n_po=35, depth=6, seed=12)
+    js = d.to_json()
+    cd, od = sim.CompiledDesign(js, meta.top), ob.OracleDesign(js, meta.top)
+    stim, rec = netlist_run_spec(meta)
+    stim = [(n, sim.STIM_RANDOM_UNIFORM if n in ("pi_1", "pi_4") else sim.STIM_TRACE if n in ("pi_2", "pi_7") else k,
+             p if n not in ("pi_2", "pi_7") else int(n == "pi_7")) for n, k, p in stim if n != "pi_5"]
+    tr = np.random.default_rng(lanes).integers(0, 1 << 32, (cycles, 2, (lanes + 31) // 32), dtype=np.uint32)
+    mode = sim.REC_TRACE | sim.REC_HASH | sim.REC_DETECT
+    g = sim.GpuBatchSimulator(cd, lanes=lanes)
+    res = g.run(cycles, seed=lanes, stim=stim, record=rec, mode=mode, input_trace=tr, lane_base=96)
+    assert g.tile_words == 0
+    ref = oracle_bp_run(od, lanes, cycles, lanes, [(od.signal(n), k, p) for n, k, p in stim], [od.signal(r) for r in rec],
+                        mode, input_trace=tr, lane_base=96)
+    for k in ("trace", "hash", "detect"):
+        assert np.array_equal(res[k], ref[k]), k
