@@ -1123,8 +1123,13 @@ const JitKernel* word_jit_for_run(rrtl_design* d, const WordRunTables& t, uint32
     });
     if (S) return S;
   }
-  const JitKernel* R = jit_cache_get(d->wjit_mu, d->wjit_runs, t.key(),
-                                   [&](JitKernel* J) { word_jit_build(d->wp, d->ctx->device, J, &t); });
+  // records hashed on a second warp (RRTL_WORD_JIT_SERVED=0: never)
+  const char* venv = getenv("RRTL_WORD_JIT_SERVED");
+  const bool served = !(venv && venv[0] == '0') && word_served_pays(d->wp, t, lanes_pad, d->ctx->sm_count, d->ctx->max_smem,
+                                                                    d->ctx->max_smem_sm);
+  const JitKernel* R = jit_cache_get(d->wjit_mu, d->wjit_runs, t.key() + (served ? "|served" : ""), [&](JitKernel* J) {
+    word_jit_build(d->wp, d->ctx->device, J, &t, nullptr, served);
+  });
   return R ? R : any;
 }
 

@@ -107,6 +107,7 @@ struct WordRunDev {
 // [row][thread] u32 words: the signal words first (when staged), then each
 // staged memory. Memories past kJitPlacedMems always stay in HBM.
 constexpr uint32_t kJitPlacedMems = 8;
+constexpr uint32_t kServedLanes = 128;  // lanes of a block whose records are hashed on other warps
 struct WordJitPlace {
   uint32_t sig_smem;      // 1: signal words staged from row 0
   uint32_t n_sig_words;

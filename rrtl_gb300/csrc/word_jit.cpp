@@ -11,6 +11,7 @@
 // slots per stream); register captures go to locals c<k> that the clock edge
 // commits after the memory writes, as the interpreter's capture buffer does.
 #include "word_jit.h"
+#include "../../include/rrtl_cuda.h"
 
 #include <dlfcn.h>
 #include <nvrtc.h>
@@ -45,10 +46,17 @@ unsigned long long wmask(uint32_t w) { return w >= 64u ? ~0ull : ((1ull << w) - 
 
 std::string u(uint64_t v) { return std::to_string(v) + "u"; }
 
+uint32_t rec_limbs(const WordRunTables& run) {
+  uint32_t n = 0;
+  for (const WordRecDev& r : run.rec) n += r.limbs;
+  return n;
+}
+
 struct Emitter {
   const WordProgram& wp;
   const WordRunTables* run = nullptr;
   const WordSplitPlan* split = nullptr;
+  bool served = false;
   std::string o;
 
   const bool regs;  // signal words as register members s<k>
@@ -527,12 +535,18 @@ struct Emitter {
       o += "  __device__ __forceinline__ static constexpr uint32_t mode() { return " + u(run->mode) + "; }\n";
       o += "};\n}  // namespace rrtl\n";
     }
-    o += std::string("extern \"C\" __global__ void __launch_bounds__(") + (split ? "64" : "128") +
+    o += std::string("extern \"C\" __global__ void __launch_bounds__(") + (split ? "64" : served ? "256" : "128") +
          ") rrtl_word_jit(const rrtl::WordRunDev R, "
          "const rrtl::WordJitPlace Pl) {\n";
     o += "  extern __shared__ uint32_t rrtl_jsm[];\n";
     if (run && split) {
       o += "  rrtl::word_jit_run_split<rrtl::JitLane>(R, Pl, rrtl_jsm, rrtl::RunSpec{});\n";
+    } else if (run && served) {
+      const uint32_t cycles = word_served_cycles(*run), limbs = rec_limbs(*run);
+      o += "  __shared__ uint32_t rows[2 * " + u(cycles) + " * " + u(limbs) + " * rrtl::kServedLanes];\n";
+      o += "  __shared__ unsigned long long sums[4 * " + u(cycles) + "];\n";
+      o += "  rrtl::word_jit_run_served<rrtl::JitLane, rrtl::RunSpec, " + u(cycles) + ", " + u(limbs) +
+           ">(R, Pl, rrtl_jsm, rrtl::RunSpec{}, rows, sums);\n";
     } else if (run) {
       o += "  rrtl::word_jit_run<rrtl::JitLane>(R, Pl, rrtl_jsm, rrtl::RunSpec{});\n";
     } else {
@@ -594,9 +608,42 @@ JitKernel::~JitKernel() {
   if (lib) cudaLibraryUnload(lib);
 }
 
-std::string word_jit_source(const WordProgram& wp, const WordRunTables* run, const WordSplitPlan* split) {
+uint32_t word_served_cycles(const WordRunTables& run) {
+  if (!(run.mode & RRTL_REC_HASH) || (run.mode & (RRTL_REC_DETECT | RRTL_REC_CHECK)) || run.rec.empty()) return 0;
+  const uint32_t n = rec_limbs(run);  // 1 KB a cycle and word: rows of at most 24 KB
+  return n <= 3 ? 8 : n <= 6 ? 4 : n <= 12 ? 2 : n <= 24 ? 1 : 0;
+}
+
+bool word_served_pays(const WordProgram& wp, const WordRunTables& run, uint32_t lanes_pad, uint32_t sm_count,
+                      size_t max_smem_block, size_t max_smem_sm) {
+  const uint32_t cycles = word_served_cycles(run), limbs = rec_limbs(run);
+  if (!cycles || !lanes_pad) return false;
+  const uint32_t blocks = lanes_pad / kServedLanes;
+  if (blocks > sm_count && wp.code.size() > 100u * (size_t)limbs) return false;
+  // memories staged beside the rows and without them (word_jit_place's order and shares)
+  std::vector<uint64_t> mems;
+  for (size_t k = 0; k < std::min<size_t>(wp.mems.size(), kJitPlacedMems); ++k)
+    mems.push_back((uint64_t)wp.mems[k].depth * wp.mems[k].limbs * kServedLanes * 4);
+  std::sort(mems.begin(), mems.end());
+  const uint32_t per_sm = std::max<uint32_t>(1, std::min<uint32_t>(4, (blocks + sm_count - 1) / std::max<uint32_t>(sm_count, 1)));
+  const size_t share = std::min(max_smem_block, max_smem_sm / per_sm);
+  auto staged = [&](size_t reserve) {
+    size_t used = reserve, n = 0;
+    for (uint64_t m : mems)
+      if (used + m <= share) {
+        used += m;
+        ++n;
+      }
+    return n;
+  };
+  const size_t rows = (size_t)2 * cycles * limbs * kServedLanes * 4 + 32 * cycles;
+  return staged(1024 + rows) == staged(1024);
+}
+
+std::string word_jit_source(const WordProgram& wp, const WordRunTables* run, const WordSplitPlan* split, bool served) {
   Emitter e(wp);
   e.run = run;
+  e.served = run && !split && served && word_served_cycles(*run);
   e.split = run ? split : nullptr;
   return e.source();
 }
@@ -852,7 +899,7 @@ void jit_build_kernel(const std::string& src, int device, const char* name, JitK
 }
 
 void word_jit_build(const WordProgram& wp, int device, JitKernel* J, const WordRunTables* run,
-                    const WordSplitPlan* split) {
+                    const WordSplitPlan* split, bool served) {
   J->written.assign(wp.mems.size(), 0);
   J->reg_signals = wp.n_sig_words <= kJitRegSignals;
   for (const WInstr& I : wp.code)
@@ -865,7 +912,8 @@ void word_jit_build(const WordProgram& wp, int device, JitKernel* J, const WordR
     J->split = true;
     J->n_xwords = (uint32_t)split->xwords.size();
   }
-  jit_build_kernel(word_jit_source(wp, run, split), device, "rrtl_word_jit", J);
+  J->served = run && !split && served && word_served_cycles(*run);
+  jit_build_kernel(word_jit_source(wp, run, split, served), device, "rrtl_word_jit", J);
 }
 
 size_t word_jit_place(const WordProgram& wp, const JitKernel& J, uint32_t n_sig_words, uint32_t lanes_pad, uint64_t cycles,
@@ -921,7 +969,7 @@ cudaError_t launch_word_jit(const JitKernel& J, const WordRunDev& R, const WordJ
   void* args[] = {&r, &p};
   if (J.split)  // 32 lanes per block on two warps
     return cudaLaunchKernel(reinterpret_cast<const void*>(J.fn), dim3(R.lanes_pad / 32u), dim3(64), args, smem, st);
-  return cudaLaunchKernel(reinterpret_cast<const void*>(J.fn), dim3(R.lanes_pad / 128u), dim3(128), args, smem, st);
+  return cudaLaunchKernel(reinterpret_cast<const void*>(J.fn), dim3(R.lanes_pad / 128u), dim3(J.served ? 256 : 128), args, smem, st);
 }
 
 }  // namespace rrtl

@@ -48,6 +48,20 @@ struct WordSplitPlan {
   size_t sizes[2] = {0, 0};
 };
 
+// Cycles of recorded words that fit the rows of a kernel whose record stage
+// runs on a second warp (word_jit_run_served); 0: the run's records do not
+// suit it (no hash, detection or checks, too many words).
+uint32_t word_served_cycles(const WordRunTables& run);
+// Whether a run of lanes_pad lanes uses that form. With a block an SM to
+// itself the recording warps cost nothing but their shared memory: it does
+// unless that would push a memory out of it. With more lanes they take
+// registers from other compute warps: only for programs whose hash is a large
+// part (at most 100 instructions per recorded word). ns per cycle, one warp /
+// two: pipelined CPU (3 words) 502 / 299 at 16,384 lanes, 752 / 549 at
+// 32,768, 2,270 / 1,845 at 131,072; Counter 234 / 104 and 775 / 516.
+bool word_served_pays(const WordProgram& wp, const WordRunTables& run, uint32_t lanes_pad, uint32_t sm_count,
+                      size_t max_smem_block, size_t max_smem_sm);
+
 // Split plan of `wp` for `run`; false (with the reason) when the design does
 // not split: asynchronous resets, combinational feedback, signals beyond the
 // register limit, or partitions too uneven to gain.
@@ -67,6 +81,7 @@ struct JitKernel {
   size_t static_smem = 0;        // the kernel's static shared memory (stimulus/record tables)
   bool reg_signals = false;      // signal words live in registers (no signal staging)
   bool split = false;            // two warps per 32 lanes (word_jit_run_split)
+  bool served = false;           // four recording warps beside four compute warps (word_jit_run_served)
   uint32_t n_xwords = 0;         // register words exchanged between the two warps
   std::vector<uint8_t> written;  // per memory: the design writes it
   ~JitKernel();
@@ -80,7 +95,7 @@ constexpr uint32_t kJitRegSignals = 256;
 // CUDA C++ source of a word program's compiled kernel `rrtl_word_jit`: for
 // any run, or with `run` for that run's tables only.
 std::string word_jit_source(const WordProgram& wp, const WordRunTables* run = nullptr,
-                            const WordSplitPlan* split = nullptr);
+                            const WordSplitPlan* split = nullptr, bool served = false);
 
 // Compile `src` for `arch` (e.g. "sm_103a") with NVRTC; returns the cubin,
 // or an empty vector with `log` holding the compiler's messages.
@@ -98,7 +113,7 @@ void jit_build_kernel(const std::string& src, int device, const char* name, JitK
 // Emit, compile and load the kernel of `wp` on the current device. Never
 // throws: failures leave ok = false and the reason in error.
 void word_jit_build(const WordProgram& wp, int device, JitKernel* out, const WordRunTables* run = nullptr,
-                    const WordSplitPlan* split = nullptr);
+                    const WordSplitPlan* split = nullptr, bool served = false);
 
 // Shared-memory placement for one launch over `lanes_pad` lanes and `cycles`
 // cycles; returns the dynamic shared memory bytes per 128-lane block.

@@ -177,15 +177,11 @@ struct JitDynamicRun {
   }
 };
 
-// Kernel body of a compiled design: stage in, run the cycles, stage out.
-// `spec` is a WordRunSpec over tables that `tables` filled, or a type whose
-// tables are compile-time constants.
-template <class L, class S>
-__device__ __forceinline__ void word_jit_run(const WordRunDev& R, const WordJitPlace& Pl, uint32_t* jsm, const S& spec) {
-  const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t T = blockDim.x;
-  uint32_t* my = jsm + threadIdx.x;
-  L W;
+// A lane's signals and memories into registers and shared memory rows (`my`:
+// the lane's column, rows of T words), and back.
+template <class L>
+__device__ __forceinline__ void jit_stage_in(const WordRunDev& R, const WordJitPlace& Pl, uint32_t* my, uint32_t T,
+                                             uint32_t lane, L& W) {
   W.LP = R.lanes_pad;
   W.gm = R.mems + lane;
   if constexpr (L::kRegSignals) {
@@ -212,8 +208,11 @@ __device__ __forceinline__ void word_jit_run(const WordRunDev& R, const WordJitP
       W.ms[k] = R.lanes_pad;
     }
   }
-  __syncthreads();  // shared-memory run tables are in place
-  word_lane_cycles(R, lane, W, spec);
+}
+
+template <class L>
+__device__ __forceinline__ void jit_stage_out(const WordRunDev& R, const WordJitPlace& Pl, const uint32_t* my, uint32_t T,
+                                              uint32_t lane, const L& W) {
   if constexpr (L::kRegSignals) {
     W.store(R.values + lane, R.lanes_pad);
   } else if (Pl.sig_smem) {
@@ -227,6 +226,147 @@ __device__ __forceinline__ void word_jit_run(const WordRunDev& R, const WordJitP
     const uint32_t* s = my + (size_t)Pl.smem_row[k] * T;
     for (uint32_t w = 0; w < Pl.mem_words[k]; ++w) g[(size_t)w * R.lanes_pad] = s[(size_t)w * T];
   }
+}
+
+// Kernel body of a compiled design: stage in, run the cycles, stage out.
+// `spec` is a WordRunSpec over tables that `tables` filled, or a type whose
+// tables are compile-time constants.
+template <class L, class S>
+__device__ __forceinline__ void word_jit_run(const WordRunDev& R, const WordJitPlace& Pl, uint32_t* jsm, const S& spec) {
+  const uint32_t lane = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t* my = jsm + threadIdx.x;
+  L W;
+  jit_stage_in(R, Pl, my, blockDim.x, lane, W);
+  __syncthreads();  // shared-memory run tables are in place
+  word_lane_cycles(R, lane, W, spec);
+  jit_stage_out(R, Pl, my, blockDim.x, lane, W);
+}
+
+// ---- recording on a second warp
+//
+// For lane counts that leave warp schedulers idle, a block of 128 lanes gets
+// four more warps that hash what the first four record: a compute warp puts
+// its recorded words of kServedCycles cycles into shared memory rows, and
+// while it fills the other half of the rows its partner turns them into hash
+// terms (one barrier of the two warps per half). A one-warp lane is bound by
+// the latency of its own instructions, and with out_pc and out_acc hashed
+// some 150 of the pipelined CPU's 403 a cycle were the hash (502 -> 299 ns a cycle at
+// 16,384 lanes; 226 without records).
+__device__ __forceinline__ void served_pair_barrier(uint32_t warp) {
+  __syncwarp();
+  asm volatile("bar.sync %0, 64;" ::"r"(1u + warp) : "memory");
+}
+
+// Recorded words of one cycle: into row `row` ([limb][lane]) and the trace.
+template <class L, class S>
+__device__ __forceinline__ void served_record(const WordRunDev& R, uint32_t lane, L& W, const S& spec, uint32_t* row,
+                                              unsigned long long c, bool live) {
+#pragma unroll
+  for (uint32_t k = 0; k < spec.n_rec(); ++k) {
+    const WordRecDev rc = spec.rec(k);
+    for (uint32_t l = 0; l < rc.limbs; ++l) {
+      uint32_t v = W.get(rc.sig_off + l);
+      if (l + 1 == rc.limbs && (rc.width & 31u)) v &= (1u << (rc.width & 31u)) - 1u;
+      row[(rc.base + l) * kServedLanes] = v;
+      if ((spec.mode() & RRTL_REC_TRACE) && live) R.out_trace[((size_t)c * R.rec_limbs + rc.base + l) * R.lanes + lane] = v;
+    }
+  }
+}
+
+// The partner warp: hash terms of every cycle, each half's sums added to the
+// run's hashes by one instruction of kCycles atomics. Its chain a cycle (salt,
+// two multiplies a term, five reduction steps) is longer than a small
+// design's cycle, so kStep cycles go side by side, share the reduction (a
+// butterfly that halves the cycles a lane holds) and, where lanes allow, one
+// salt evaluation serves the whole half.
+template <class S, uint32_t kCycles, uint32_t kLimbs>
+__device__ __forceinline__ void served_hash(const WordRunDev& R, uint32_t lane, const S& spec, const uint32_t* rows,
+                                            unsigned long long* sums, uint32_t warp) {
+  constexpr uint32_t kStep = kCycles < 4u ? kCycles : 4u, kRec = S::n_rec();
+  constexpr bool kHalfSalts = kRec * kCycles <= 32u;
+  const bool live = lane < R.lanes;
+  const uint32_t wl = threadIdx.x & 31u;
+  for (unsigned long long c0 = 0; c0 < R.cycles; c0 += kCycles) {
+    const uint32_t n = R.cycles - c0 < kCycles ? (uint32_t)(R.cycles - c0) : kCycles;
+    const uint32_t* half = rows + ((c0 / kCycles) & 1u) * (kCycles * kLimbs * kServedLanes);
+    unsigned long long salts = kHalfSalts ? hash_salt(R.cycle_base + c0 + wl / kRec, wl % kRec) : 0ull;
+    served_pair_barrier(warp);  // the half is filled
+#pragma unroll 1
+    for (uint32_t j0 = 0; j0 < n; j0 += kStep) {
+      unsigned long long h[kStep];
+#pragma unroll
+      for (uint32_t j = 0; j < kStep; ++j) {  // (cycles past the run's end sum rows nothing wrote, and are not added)
+        h[j] = 0ull;
+#pragma unroll
+        for (uint32_t k = 0; k < kRec; ++k) {
+          const WordRecDev rc = spec.rec(k);
+          if (!kHalfSalts && (k & 31u) == 0) salts = hash_salt(R.cycle_base + c0 + j0 + j, k + wl);
+          const unsigned long long salt = __shfl_sync(0xFFFFFFFFu, salts, kHalfSalts ? (j0 + j) * kRec + k : k & 31u);
+          for (uint32_t l = 0; l < rc.limbs; ++l) {
+            const uint32_t v = half[((j0 + j) * kLimbs + rc.base + l) * kServedLanes];
+            if (rc.width == 1) {
+              // 1-bit signals hash as 32-lane packed words, the gate engine's unit
+              const uint32_t packed = __ballot_sync(0xFFFFFFFFu, live && (v & 1u));
+              if (wl == 0 && live) h[j] += hash_term_salted(salt, (R.lane_base + lane) >> 5, packed);
+            } else {
+              const unsigned long long t = hash_term_salted(salt, (R.lane_base + lane) * rc.limbs + l, v);
+              h[j] += live ? t : 0ull;
+            }
+          }
+        }
+      }
+      // lane bits 4 and 3 choose the cycle a lane ends up with
+      uint32_t mine = 0, bit = 16;
+#pragma unroll
+      for (uint32_t m = kStep / 2; m >= 1u; m /= 2, bit /= 2) {
+        const bool up = wl & bit;
+#pragma unroll
+        for (uint32_t j = 0; j < m; ++j) {
+          const unsigned long long give = up ? h[j] : h[j + m], keep = up ? h[j + m] : h[j];
+          h[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, bit);
+        }
+        mine += up ? m : 0u;
+      }
+      for (uint32_t o = bit; o > 0; o >>= 1) h[0] += __shfl_xor_sync(0xFFFFFFFFu, h[0], o);
+      if ((wl & (2u * bit - 1u)) == 0u) sums[j0 + mine] = h[0];
+    }
+    __syncwarp();
+    if (wl < n && sums[wl]) atomicAdd(R.out_hash + c0 + wl, sums[wl]);
+    __syncwarp();
+  }
+}
+
+// rows: [2][kCycles][kLimbs][128]; sums: [4][kCycles].
+template <class L, class S, uint32_t kCycles, uint32_t kLimbs>
+__device__ __forceinline__ void word_jit_run_served(const WordRunDev& R, const WordJitPlace& Pl, uint32_t* jsm, const S& spec,
+                                                    uint32_t* rows, unsigned long long* sums) {
+  const uint32_t tl = threadIdx.x % kServedLanes, warp = tl >> 5;
+  const uint32_t lane = blockIdx.x * kServedLanes + tl;
+  if (threadIdx.x >= kServedLanes) {
+    served_hash<S, kCycles, kLimbs>(R, lane, spec, rows + tl, sums + warp * kCycles, warp);
+    return;
+  }
+  uint32_t* my = jsm + tl;
+  L W;
+  jit_stage_in(R, Pl, my, kServedLanes, lane, W);
+  const bool live = lane < R.lanes;
+  if (R.start_settle) W.settle();
+  uint32_t at = 0;  // cycle within the rows
+  for (unsigned long long c = 0; c < R.cycles; ++c) {
+    word_stimulus(R, lane, W, spec, c, R.cycle_base + c, live);
+    W.settle();
+    served_record(R, lane, W, spec, rows + tl + at * (kLimbs * kServedLanes), c, live);
+    W.edge();
+    ++at;
+    if (at == kCycles) served_pair_barrier(warp);
+    if (at == 2 * kCycles) {
+      served_pair_barrier(warp);
+      at = 0;
+    }
+  }
+  if (at % kCycles) served_pair_barrier(warp);
+  if (R.final_settle) W.settle();
+  jit_stage_out(R, Pl, my, kServedLanes, lane, W);
 }
 
 // ---- two-warp split of a compiled kernel

@@ -195,3 +195,38 @@ def test_random_designs_two_warp_split(engine, monkeypatch, seed):
     stim += [(n, sim.STIM_RANDOM, i + 7) for i, (n, w) in enumerate(meta["inputs"])]
     rec = [n for n, w in meta["outputs"]]
     _split_vs_unsplit(monkeypatch, d.to_json(), meta["top"], 100, 30, stim, rec, sim.REC_TRACE | sim.REC_HASH)
+
+
+@pytest.mark.parametrize("widths", [(1, 2), (8, 1, 32), (40, 1, 64), (64, 33, 7, 96, 1, 31), (64,) * 9 + (5,), (64,) * 13])
+@pytest.mark.parametrize("lanes,cycles", [(1, 1), (129, 7), (128, 8), (300, 9), (40, 17), (260, 32)])
+def test_records_on_a_second_warp(engine, widths, lanes, cycles):
+    """Hashes of records of every row shape (8, 4, 2 and 1 cycles a half, and
+    more words than the rows take), around the halves and the 128-lane blocks."""
+    from rrtl_gb300.builder import Design, uint
+
+    d = Design()
+    m = d.module("W")
+    clk, rst = m.input("clk", uint(1)), m.input("rst", uint(1))
+    rec = []
+    for i, w in enumerate(widths):
+        x, r, o = m.input(f"x{i}", uint(w)), m.reg(f"r{i}", uint(w)), m.output(f"o{i}", uint(w))
+        m.clock(r, clk)
+        m.reset(r, rst, 0)
+        m.next(r, (r + x) if w > 1 else (r ^ x))
+        m.assign(o, r ^ x)
+        rec.append(f"o{i}")
+    js = d.to_json()
+    stim = [("clk", sim.STIM_CONST, 1), ("rst", sim.STIM_PULSE, 1)] + [(f"x{i}", sim.STIM_RANDOM, i) for i in range(len(widths))]
+    od = ob.OracleDesign(js, "W")
+    g = sim.GpuBatchSimulator(js, "W", lanes)
+    mode = sim.REC_HASH | sim.REC_TRACE
+    res = g.run(cycles, seed=6, stim=stim, record=rec, mode=mode)
+    ref = oracle_packed_run(od, lanes, cycles, 6, [(od.signal(n), k, p) for n, k, p in stim], [od.signal(r) for r in rec], 3)
+    assert np.array_equal(res["trace"], ref["trace"]) and np.array_equal(res["hash"], ref["hash"])
+    # a second run goes on from the state, on the hash alone
+    res = g.run(cycles, seed=8, stim=stim[2:], record=rec, mode=sim.REC_HASH)
+    f = sim.GpuBatchSimulator(js, "W", lanes)
+    f.set_path(sim.PATH_WORD_INTERP)
+    f.run(cycles, seed=6, stim=stim, record=rec, mode=mode)
+    assert np.array_equal(res["hash"], f.run(cycles, seed=8, stim=stim[2:], record=rec, mode=sim.REC_HASH)["hash"])
+    assert all(np.array_equal(a, b) for a, b in zip(g.snapshot_storage(), f.snapshot_storage()))
