@@ -511,6 +511,8 @@ struct Timer {
   void stop() { cuda_check(cudaEventRecord(b->ev1, b->d->ctx->stream), "event"); }
 };
 
+// The batch's device status word, read by the same synchronisation as the
+// copies issued before it.
 void check_err_word(rrtl_batch* b) {
   uint32_t e = 0;
   cuda_check(cudaMemcpyAsync(&e, b->d_err.p, 4, cudaMemcpyDeviceToHost, b->d->ctx->stream), "err");
@@ -1579,8 +1581,7 @@ void batch_tick_many(rrtl_batch* b, uint64_t steps, bool sync) {
   rrtl_run r{};
   r.cycles = steps;
   if (b->d->engine == RRTL_ENGINE_GATE) gate_run(b, r, !sync);
-  else word_run(b, r, !sync, true, true);
-  if (sync) check_err_word(b);
+  else word_run(b, r, !sync, true, true);  // (a synchronous run checks the error word itself)
 }
 
 }  // namespace rrtl
@@ -2166,7 +2167,7 @@ static void gate_get_bits(rrtl_batch* b, uint32_t signal, uint32_t* words) {
   cuda_check(cudaMemcpyAsync(words, b->d_nets.as<uint32_t>() + (size_t)net * b->words_pad, (size_t)b->words * 4,
                              cudaMemcpyDeviceToHost, b->d->ctx->stream),
              "d2h signal");
-  cuda_check(cudaStreamSynchronize(b->d->ctx->stream), "sync");
+  check_err_word(b);
   uint32_t valid = b->lanes - (b->words - 1) * 32;
   if (valid < 32) words[b->words - 1] &= (1u << valid) - 1u;
 }
@@ -2206,7 +2207,6 @@ rrtl_status rrtl_batch_get_signal_limbs(rrtl_batch* b, uint32_t signal, uint32_t
     set_device(b->d->ctx);
     const PackedSignal& ps = signal_of(b->d, signal);
     REQUIRE(n == (size_t)ps.layout.limbs * b->lanes, RRTL_E_ARG, "E_GPU_LANE_VALUES: output size mismatch");
-    check_err_word(b);
     if (b->d->engine == RRTL_ENGINE_GATE) {
       std::vector<uint32_t> words(b->words);
       gate_get_bits(b, signal, words.data());
@@ -2217,7 +2217,7 @@ rrtl_status rrtl_batch_get_signal_limbs(rrtl_batch* b, uint32_t signal, uint32_t
       cuda_check(cudaMemcpyAsync(rows.data(), b->d_values.as<uint32_t>() + (size_t)ps.layout.offset * b->lanes_pad,
                                  rows.size() * 4, cudaMemcpyDeviceToHost, b->d->ctx->stream),
                  "d2h signal");
-      cuda_check(cudaStreamSynchronize(b->d->ctx->stream), "sync");
+      check_err_word(b);
       for (uint32_t k = 0; k < limbs; ++k)
         for (uint32_t l = 0; l < b->lanes; ++l) {
           uint32_t v = rows[(size_t)k * b->lanes_pad + l];
@@ -2253,7 +2253,6 @@ rrtl_status rrtl_batch_get_signal_bits(rrtl_batch* b, uint32_t signal, uint32_t*
     const PackedSignal& ps = signal_of(b->d, signal);
     REQUIRE(ps.layout.width == 1, RRTL_E_ARG, "E_GPU_WIDE_SIGNAL: bit-packed access needs a 1-bit signal");
     REQUIRE(n == (b->lanes + 31) / 32, RRTL_E_ARG, "E_GPU_LANE_VALUES: expected ceil(lanes/32) words");
-    check_err_word(b);
     if (b->d->engine == RRTL_ENGINE_GATE) {
       gate_get_bits(b, signal, out);
     } else {
@@ -2274,7 +2273,6 @@ rrtl_status rrtl_batch_get_signals_bits(rrtl_batch* b, const uint32_t* signals, 
     REQUIRE(n_out == n * words, RRTL_E_ARG, "E_GPU_LANE_VALUES: expected n*ceil(lanes/32) words");
     for (size_t i = 0; i < n; ++i)
       REQUIRE(signal_of(b->d, signals[i]).layout.width == 1, RRTL_E_ARG, "E_GPU_WIDE_SIGNAL: bit-packed access needs 1-bit signals");
-    check_err_word(b);
     if (b->d->engine == RRTL_ENGINE_GATE) {
       cudaStream_t st = b->d->ctx->stream;
       // one 2-D copy per run of consecutive net rows
@@ -2287,7 +2285,7 @@ rrtl_status rrtl_batch_get_signals_bits(rrtl_batch* b, const uint32_t* signals, 
                    "d2h signals");
         i = j;
       }
-      cuda_check(cudaStreamSynchronize(st), "sync");
+      check_err_word(b);
       uint32_t valid = b->lanes - (words - 1) * 32;
       if (valid < 32)
         for (size_t i = 0; i < n; ++i) out[i * words + words - 1] &= (1u << valid) - 1u;
@@ -2336,12 +2334,11 @@ rrtl_status rrtl_batch_get_memory_limbs(rrtl_batch* b, uint32_t memory, uint32_t
     uint32_t limbs = m.data_layout.limbs;
     size_t words = (size_t)m.depth * limbs;
     REQUIRE(n == words * b->lanes, RRTL_E_ARG, "E_GPU_MEMORY_VALUES: expected depth*limbs*lanes values");
-    check_err_word(b);
     std::vector<uint32_t> rows(words * b->lanes_pad);
     cuda_check(cudaMemcpyAsync(rows.data(), b->d_mem.as<uint32_t>() + (size_t)m.offset * b->lanes_pad, rows.size() * 4,
                                cudaMemcpyDeviceToHost, b->d->ctx->stream),
                "d2h memory");
-    cuda_check(cudaStreamSynchronize(b->d->ctx->stream), "sync");
+    check_err_word(b);
     for (size_t wv = 0; wv < words; ++wv)
       for (uint32_t l = 0; l < b->lanes; ++l) {
         uint32_t v = rows[wv * b->lanes_pad + l];

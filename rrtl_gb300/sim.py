@@ -53,6 +53,10 @@ class Stim(ctypes.Structure):
     _fields_ = [("signal", c_uint32), ("kind", c_uint32), ("param", c_uint64)]
 
 
+_STIM_DTYPE = np.dtype([("signal", np.uint32), ("kind", np.uint32), ("param", np.uint64)])  # Stim's layout
+assert _STIM_DTYPE.itemsize == ctypes.sizeof(Stim)
+
+
 class Run(ctypes.Structure):
     _fields_ = [
         ("cycles", c_uint64),
@@ -489,12 +493,33 @@ class CompiledDesign:
         check(load(self.ctx.h, raw, len(raw), top.encode(), byref(self.h)))
         self.top = top
         self._cache = {}
+        self._engine = None
 
     @property
     def info(self) -> DesignInfo:
         i = DesignInfo()
         check(lib().rrtl_design_info_get(self.h, byref(i)))
         return i
+
+    @property
+    def engine(self) -> int:
+        """ENGINE_GATE or ENGINE_WORD."""
+        if self._engine is None:
+            self._engine = self.info.engine
+        return self._engine
+
+    def indices(self, signals) -> np.ndarray:
+        """Packed indices of signals given by name (or index)."""
+        cache = self._cache
+        out = []
+        for s in signals:
+            if isinstance(s, str):
+                out.append((cache.get(s) or self.signal(s))[0])
+            elif isinstance(s, int):
+                out.append(s & 0xFFFFFFFF)
+            else:
+                raise TypeError("signals are addressed by name or packed index")
+        return np.array(out, dtype=np.uint32)
 
     def signal(self, name: str):
         """(index, width, kind) of a signal by name."""
@@ -630,9 +655,9 @@ class GpuBatchSimulator:
 
     def get_signals_bits(self, signals) -> np.ndarray:
         """[n][ceil(lanes/32)] bit-packed values of several 1-bit signals."""
-        idx = np.asarray([self._sig(s) for s in signals], dtype=np.uint32)
+        idx = self.design.indices(signals)
         words = (self.lanes + 31) // 32
-        out = np.zeros((len(idx), words), dtype=np.uint32)
+        out = np.empty((len(idx), words), dtype=np.uint32)
         check(lib().rrtl_batch_get_signals_bits(self.h, _u32p(idx), len(idx), _u32p(out), out.size))
         return out
 
@@ -705,14 +730,19 @@ class GpuBatchSimulator:
     def make_run(self, cycles: int, seed: int = 0, stim: Iterable = (), record: Iterable = (), mode: int = 0,
                  input_trace: Optional[np.ndarray] = None, out_trace=None, out_hash=None, detect=None,
                  lane_base: int = 0) -> Run:
-        st = [(self._sig(s), k, p) for (s, k, p) in stim]
-        arr = (Stim * max(1, len(st)))(*[Stim(a, b, c) for a, b, c in st])
-        rec = np.asarray([self._sig(r) for r in record], dtype=np.uint32)
+        st = list(stim)
+        arr = np.zeros(max(1, len(st)), dtype=_STIM_DTYPE)
+        if st:
+            names, kinds, params = zip(*st)
+            arr["signal"] = self.design.indices(names)
+            arr["kind"] = np.array([k & 0xFFFFFFFF for k in kinds], dtype=np.uint32)
+            arr["param"] = np.array([p & 0xFFFFFFFFFFFFFFFF for p in params], dtype=np.uint64)
+        rec = self.design.indices(record)
         r = Run()
         r.cycles = cycles
         r.seed = seed
         r.n_stim = len(st)
-        r.stim = ctypes.cast(arr, POINTER(Stim))
+        r.stim = arr.ctypes.data_as(POINTER(Stim))
         r.n_record = len(rec)
         r.record = _u32p(rec) if len(rec) else None
         r.record_mode = mode
@@ -727,21 +757,20 @@ class GpuBatchSimulator:
         r._keep = (arr, rec, input_trace, out_trace, out_hash, detect)
         return r
 
-    def alloc_outputs(self, cycles: int, record: list, mode: int) -> dict:
+    def alloc_outputs(self, cycles: int, record: list, mode: int, fill=np.zeros) -> dict:
         """Host arrays for a run's recorded outputs (None where not requested)."""
-        engine = self.design.info.engine
         words = (self.lanes + 31) // 32
         out_trace = out_hash = detect = None
         if mode & REC_TRACE:
-            if engine == ENGINE_GATE:
-                out_trace = np.zeros((cycles, len(record), words), dtype=np.uint32)
+            if self.design.engine == ENGINE_GATE:
+                out_trace = fill((cycles, len(record), words), dtype=np.uint32)
             else:
                 limbs = sum(max(1, (self.design.signal(r)[1] + 31) // 32) for r in record)
-                out_trace = np.zeros((cycles, limbs, self.lanes), dtype=np.uint32)
+                out_trace = fill((cycles, limbs, self.lanes), dtype=np.uint32)
         if mode & REC_HASH:
-            out_hash = np.zeros(cycles, dtype=np.uint64)
+            out_hash = fill(cycles, dtype=np.uint64)
         if mode & REC_DETECT:
-            detect = np.zeros(self.lanes, dtype=np.uint32)
+            detect = fill(self.lanes, dtype=np.uint32)
         return {"trace": out_trace, "hash": out_hash, "detect": detect}
 
     def run(self, cycles: int, seed: int = 0, stim: Iterable = (), record: Iterable = (), mode: int = 0,
@@ -750,7 +779,7 @@ class GpuBatchSimulator:
         lane_base: global index of this batch's lane 0 (a multiple of 32) when the batch is one shard of a
         larger run (random stimulus and hash terms follow global lanes)."""
         record = list(record)
-        out = self.alloc_outputs(cycles, record, mode)
+        out = self.alloc_outputs(cycles, record, mode, np.empty)  # the run writes every element or raises
         r = self.make_run(cycles, seed, stim, record, mode, input_trace, out["trace"], out["hash"], out["detect"],
                           lane_base)
         check(lib().rrtl_batch_run(self.h, byref(r)))
