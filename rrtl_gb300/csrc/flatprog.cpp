@@ -612,7 +612,7 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
   if (V != 4 && V != 2 && V != 1) throw RrtlError("E_GATE_SCOPE", "row vectors are 4, 2 or 1 words");
   FlatProgram fp;
   fp.V = V;
-  const uint32_t G = fp.G = 32 / V, warps = fp.warps = opt.warps;
+  const uint32_t G = fp.G = 32 / V;
   Logic lg(gp);
   lg.observe = opt.observe;
   lg.collect();
@@ -756,13 +756,17 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
 
   const bool tight = opt.max_slots != 0;
 
-  // ---- levels: group, place, schedule
+  // ---- levels: group and place
   fp.net_level.assign(gp.n_nets, -1);
   fp.net_warp.assign(gp.n_nets, 0);
   Grouper grouper{G, cells, slot};
-  std::vector<std::vector<FlatLane>> streams(warps);
-  std::vector<uint32_t> last_level(warps, 0);
   std::vector<uint8_t> used_res(G);
+  struct Entry {
+    std::vector<FlatLane> lanes;
+    std::vector<uint32_t> outs;  // nets written
+    double cost = 0;
+  };
+  std::vector<std::vector<Entry>> entries(NL);
   for (uint32_t L = 0; L < NL; ++L) {
     for (uint32_t n : q_free_at[L]) release((uint32_t)slot[n]);
     if (L > 0)
@@ -815,12 +819,7 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
         fp.floor_wavefronts += gs == &g2 ? 3 : 4;
       }
     // entries of this level: V groups fill a warp's lanes
-    struct Entry {
-      std::vector<FlatLane> lanes;
-      std::vector<uint32_t> outs;  // nets written
-      double cost = 0;
-    };
-    std::vector<Entry> es;
+    std::vector<Entry>& es = entries[L];
     auto lane_fill = [&](const std::vector<Group>& gs, size_t g0, auto&& put) {
       for (uint32_t h = 0; h < V; ++h) {
         const size_t gi = g0 + h;
@@ -879,6 +878,18 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
       e.cost = 5.0;
       es.push_back(std::move(e));
     }
+    fp.n_entries += (uint32_t)es.size();
+  }
+  // ---- schedule: as many warps as a level has entries on average. A warp
+  // without an entry in a level still spends an idle one on its barrier: 10,000
+  // gates (4.7 entries a level), clocks per tile-cycle of one-word and of
+  // 4-word tiles: 16 warps 17.7k and 27.0k, 8 14.5k and 20.9k, 6 12.5k and
+  // 17.2k, 5 12.4k and 17.4k.
+  const uint32_t warps = fp.warps = std::max(1u, std::min(opt.max_warps, NL ? (fp.n_entries + NL - 1) / NL : 1u));
+  std::vector<std::vector<FlatLane>> streams(warps);
+  std::vector<uint32_t> last_level(warps, 0);
+  for (uint32_t L = 0; L < NL; ++L) {
+    std::vector<Entry>& es = entries[L];
     // longest first onto the least loaded warp; warps rotate so that no warp is always the longest
     std::stable_sort(es.begin(), es.end(), [](const Entry& a, const Entry& b) { return a.cost > b.cost; });
     std::vector<double> load(warps, 0.0);
@@ -902,7 +913,6 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
         if (syncs) l.y |= kFlatDevSync;
         streams[w].push_back(l);
       }
-      ++fp.n_entries;
     }
   }
   if (next_slot > kMaxSlots) next_slot = kMaxSlots + 1;

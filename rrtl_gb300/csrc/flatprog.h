@@ -81,7 +81,7 @@ struct FlatOptions {
   bool pack = true;
   bool fold_regs = true;
   bool observe = false;  // every signal keeps a row of its own (stuck-at forces act on any of them)
-  uint32_t warps = kFlatComputeThreads / 32;
+  uint32_t max_warps = kFlatComputeThreads / 32;  // of the set; a program of few entries a level uses fewer
   uint32_t max_slots = 0;  // above this, a row is placed at any residue before the slot array grows (0: no limit)
 };
 

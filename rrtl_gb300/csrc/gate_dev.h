@@ -97,7 +97,7 @@ struct FlatProgDev {
   const uint32_t* src_net;
   const uint32_t* src_slot;
   const GateRegDev* commit;    // rows (kFlatConst0/1: a constant)
-  uint32_t n_src, n_commit, n_slots;
+  uint32_t n_src, n_commit, n_slots, warps;
 };
 
 struct GateRunDev {

@@ -6,24 +6,26 @@
 
 namespace rrtl {
 
-template <int V, int N, int Q, bool F>
+template <int V, int N, int Q, bool F, bool kFull>
 __global__ void __launch_bounds__(kFlatThreads, 1) gate_flat_kernel(FlatProgDev P, GateRunDev R) {
   extern __shared__ __align__(128) uint8_t smem[];
   for (uint32_t tile = blockIdx.x; tile < R.n_tiles; tile += gridDim.x)
-    flat_tile<V, N, Q, F>(P, R, tile, R.cycle_base, R.cycles, smem);
+    flat_tile<V, N, Q, F, kFull>(P, R, tile, R.cycle_base, R.cycles, smem);
 }
 
-template <int V, int N, int Q, bool F>
+template <int V, int N, int Q, bool F, bool kFull>
 static cudaError_t launch_f(const FlatProgDev& P, const GateRunDev& R, uint32_t grid, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(gate_flat_kernel<V, N, Q, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlatSmem);
+  cudaError_t e = cudaFuncSetAttribute(gate_flat_kernel<V, N, Q, F, kFull>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlatSmem);
   if (e != cudaSuccess) return e;
-  gate_flat_kernel<V, N, Q, F><<<grid, kFlatThreads, kFlatSmem, st>>>(P, R);
+  gate_flat_kernel<V, N, Q, F, kFull><<<grid, kFlatThreads, kFlatSmem, st>>>(P, R);
   return cudaGetLastError();
 }
 
 template <int V, int N, int Q>
 static cudaError_t launch(const FlatProgDev& P, const GateRunDev& R, uint32_t grid, cudaStream_t st) {
-  return R.has_forces ? launch_f<V, N, Q, true>(P, R, grid, st) : launch_f<V, N, Q, false>(P, R, grid, st);
+  if (R.has_forces) return launch_f<V, N, Q, true, false>(P, R, grid, st);
+  return P.warps == kFlatComputeThreads / 32 / Q ? launch_f<V, N, Q, false, true>(P, R, grid, st)
+                                                 : launch_f<V, N, Q, false, false>(P, R, grid, st);
 }
 
 cudaError_t launch_gate_flat(uint32_t V, uint32_t N, uint32_t Q, const FlatProgDev& P, const GateRunDev& R, uint32_t grid,
@@ -44,8 +46,8 @@ cudaError_t launch_gate_flat(uint32_t V, uint32_t N, uint32_t Q, const FlatProgD
 // descriptor lies in the header of shared memory, behind the detection state.
 template <int V, int N, int Q>
 __device__ __forceinline__ void queue_tile(const FlatJobDev& J, const GateItemDev& item, uint8_t* smem) {
-  if (J.R.has_forces) flat_tile<V, N, Q, true>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
-  else flat_tile<V, N, Q, false>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
+  if (J.R.has_forces) flat_tile<V, N, Q, true, false>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
+  else flat_tile<V, N, Q, false, false>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
 }
 
 __global__ void __launch_bounds__(kFlatThreads, 1) gate_flat_queue_kernel(FlatQueueDev L) {

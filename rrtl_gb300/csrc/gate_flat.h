@@ -132,14 +132,24 @@ __device__ __forceinline__ uint4 flat_load_entry(const uint4* p) {
   return r;
 }
 
-// Barrier between levels of one warp set (ids 2, 3), passed when `go` is not
-// zero (the same on every lane of the warp).
-template <int Q>
-__device__ __forceinline__ void flat_pass(uint32_t go, uint32_t set) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p bar.sync %1, %2;\n}\n" ::"r"(go), "r"(2u + set),
-               "n"(kFlatComputeThreads / Q)
-               : "memory");
-}
+// The barrier between levels of one warp set (ids from 2), for as many
+// threads as the program has streams; kFull is that count where it is every
+// warp of the set (as an immediate the barrier is cheaper: 2% of a
+// tile-cycle of 16 words), 0 where it is known at run time only.
+template <int kFull>
+struct FlatBar {
+  uint32_t id, threads;
+  // Passed when `go` is not zero (the same on every lane of the warp).
+  __device__ __forceinline__ void pass(uint32_t go) const {
+    if constexpr (kFull > 0)
+      asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p bar.sync %1, %2;\n}\n" ::"r"(go), "r"(id), "n"(kFull)
+                   : "memory");
+    else
+      asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p bar.sync %1, %2;\n}\n" ::"r"(go), "r"(id), "r"(threads)
+                   : "memory");
+  }
+};
+
 __device__ __forceinline__ void flat_bar_service() {
   __syncwarp();
   asm volatile("bar.sync 1, %0;" ::"n"(kFlatServiceThreads) : "memory");
@@ -156,8 +166,8 @@ __device__ __forceinline__ const typename FlatVec<V>::T* flat_row(const uint8_t*
 // other's rows, so every load of an entry may precede its stores (which the
 // compiler cannot know). Functions and row addresses are decoded before the
 // level barrier the entry may wait for.
-template <int V, int N, int Q>
-__device__ __forceinline__ void flat_pair2(uint8_t* S, const uint4& r, uint32_t go, uint32_t set) {
+template <int V, int N, int Q, class Bar>
+__device__ __forceinline__ void flat_pair2(uint8_t* S, const uint4& r, uint32_t go, const Bar& bar) {
   using T = typename FlatVec<V>::T;
   constexpr uint32_t kStep = flat_plane_bytes(N * Q) / sizeof(T);
   constexpr int H = N > 2 ? 2 : N;  // planes whose operands are in registers at once
@@ -168,7 +178,7 @@ __device__ __forceinline__ void flat_pair2(uint8_t* S, const uint4& r, uint32_t 
   const T* const pd = flat_row<V>(S, r.z >> 16);
   T* const po = const_cast<T*>(flat_row<V>(S, r.y & 0xFFFFu));
   T* const pq = const_cast<T*>(flat_row<V>(S, r.w & 0xFFFFu));
-  flat_pass<Q>(go, set);
+  bar.pass(go);
 #pragma unroll
   for (int p0 = 0; p0 < N; p0 += H) {
     T a[H], b[H], c[H], d[H];
@@ -189,8 +199,8 @@ __device__ __forceinline__ void flat_pair2(uint8_t* S, const uint4& r, uint32_t 
   }
 }
 
-template <int V, int N, int Q>
-__device__ __forceinline__ void flat_one3(uint8_t* S, const uint4& r, uint32_t go, uint32_t set) {
+template <int V, int N, int Q, class Bar>
+__device__ __forceinline__ void flat_one3(uint8_t* S, const uint4& r, uint32_t go, const Bar& bar) {
   using T = typename FlatVec<V>::T;
   constexpr uint32_t kStep = flat_plane_bytes(N * Q) / sizeof(T);
   constexpr int H = N > 2 ? 2 : N;
@@ -199,7 +209,7 @@ __device__ __forceinline__ void flat_one3(uint8_t* S, const uint4& r, uint32_t g
   const T* const pb = flat_row<V>(S, r.x >> 16);
   const T* const pc = flat_row<V>(S, r.z);
   T* const po = const_cast<T*>(flat_row<V>(S, r.y & 0xFFFFu));
-  flat_pass<Q>(go, set);
+  bar.pass(go);
 #pragma unroll
   for (int p0 = 0; p0 < N; p0 += H) {
     T a[H], b[H], c[H];
@@ -262,14 +272,14 @@ struct FlatForces {
 
 __device__ __forceinline__ void flat_bar_compute() {
   __syncwarp();
-  asm volatile("bar.sync 4, %0;" ::"n"(kFlatComputeThreads) : "memory");
+  asm volatile("bar.sync 6, %0;" ::"n"(kFlatComputeThreads) : "memory");
 }
 
 // Cycles [c0, c0 + ncyc) of one tile (V * N * Q words) of a run; F: with
-// stuck-at forces. Source nets are
-// read from and written back to the run's global rows; the caller settles the
-// other nets (the closing settle) afterwards.
-template <int V, int N, int Q, bool F>
+// stuck-at forces; kFull: the program has a stream for every warp of a set.
+// Source nets are read from and written back to the run's global rows; the
+// caller settles the other nets (the closing settle) afterwards.
+template <int V, int N, int Q, bool F, bool kFull>
 __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev& R, uint32_t tile, uint64_t c0,
                                           uint64_t ncyc, uint8_t* smem) {
   constexpr uint32_t W = V * N * Q;
@@ -303,16 +313,18 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
     constexpr uint32_t kSetWarps = kFlatComputeThreads / 32 / Q;
     const uint32_t set = Q == 1 ? 0u : tid / (kFlatComputeThreads / Q), warp = (tid >> 5) % kSetWarps;
     uint8_t* const Sq = S + set * (N * kPlane);  // the set's planes
-    const uint32_t begin = __ldg(P.warp_begin + warp), n = __ldg(P.warp_begin + warp + 1) - begin;
-    const uint32_t tail = __ldg(P.warp_tail + warp);
+    const FlatBar<kFull ? (int)(kFlatComputeThreads / Q) : 0> bar{2u + set, P.warps * 32u};
+    const bool active = warp < P.warps;  // a program of few cells a level has fewer streams than the set has warps
+    const uint32_t begin = active ? __ldg(P.warp_begin + warp) : 0u, n = active ? __ldg(P.warp_begin + warp + 1) - begin : 0u;
+    const uint32_t tail = active ? __ldg(P.warp_tail + warp) : 0u;
     const uint4* const base = P.stream + (size_t)begin * 32u + lane;
     FlatForces forces{};
     uint32_t begin0 = 0, end0 = 0;  // forces of registers; the thread's first stays in registers
     uint4 first0{};
     if constexpr (F) {
-      const uint32_t k = tile * (Q * kSetWarps) + (tid >> 5);
-      forces.base = R.flat_forces + __ldg(R.flat_off + k);
-      forces.n = __ldg(R.flat_off + k + 1) - __ldg(R.flat_off + k);
+      const uint32_t k = (tile * Q + set) * P.warps + warp;
+      forces.base = R.flat_forces + (active ? __ldg(R.flat_off + k) : 0u);
+      forces.n = active ? __ldg(R.flat_off + k + 1) - __ldg(R.flat_off + k) : 0u;
       forces.begin(lane, true);
       begin0 = __ldg(R.flat_off0 + tile);
       end0 = __ldg(R.flat_off0 + tile + 1);
@@ -338,8 +350,8 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
             if (go) forces.apply(S, level, lane);  // the same on every lane
           }
           // (the vote makes the branch a warp-uniform one)
-          if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, Q>(Sq, r, go, set);
-          else flat_pair2<V, N, Q>(Sq, r, go, set);
+          if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, Q>(Sq, r, go, bar);
+          else flat_pair2<V, N, Q>(Sq, r, go, bar);
           if constexpr (F) {
             if (go) forces.advance(level++);
           }
@@ -349,7 +361,7 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
       }
       for (uint32_t k = tail; k; --k) {
         if constexpr (F) forces.apply(S, level, lane);
-        flat_pass<Q>(1u, set);
+        bar.pass(1u);
         if constexpr (F) forces.advance(level++);
       }
       if constexpr (F) forces.apply(S, level, lane);

@@ -281,7 +281,7 @@ GateVariant* gate_variant(rrtl_design* d, uint32_t W) {
 // with a row for every signal (runs with stuck-at forces).
 FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe) {
   std::lock_guard<std::mutex> lk(d->gvar_mu);
-  std::unique_ptr<FlatVariant>& slot = d->fvar[log2_words(V)][Q - 1][observe ? 1 : 0];
+  std::unique_ptr<FlatVariant>& slot = d->fvar[log2_words(V)][log2_words(Q)][observe ? 1 : 0];
   if (slot) return slot.get();
   auto v = std::make_unique<FlatVariant>();
   const GateProgram& gp = d->gp();
@@ -293,7 +293,7 @@ FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe) 
     return slots <= kMaxSlots && d->ctx->max_smem >= kFlatSmem ? n : 0u;
   };
   FlatOptions o;
-  o.warps = kFlatComputeThreads / 32 / Q;
+  o.max_warps = kFlatComputeThreads / 32 / Q;
   o.observe = observe;
   v->fp = build_flat_program(gp, V, o);
   v->max_n = fit(v->fp.n_slots);
@@ -337,6 +337,7 @@ FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe) 
     P.n_src = (uint32_t)fp.source_nets.size();
     P.n_commit = (uint32_t)commit.size();
     P.n_slots = fp.n_slots;
+    P.warps = fp.warps;
   }
   slot = std::move(v);
   return slot.get();
@@ -406,13 +407,15 @@ uint32_t choose_tile_words(rrtl_design* d, uint32_t words) {
 // explicit tile width. RRTL_FLAT=0 keeps the fused kernel and RRTL_FLAT=VNQ
 // forces a shape (A/B switches).
 //
-// The cost of a tile-cycle in SM clocks was measured on the 50,000-gate
-// netlist (41 levels, 860 entries, 17,700 wavefronts per 4-word vector), one
-// wave of tiles: 25.1k at one-word rows, 29.0k at two, and 37.5k / 56.4k /
-// 79.0k / 98.2k for one to four 4-word vectors (four of them as two warp sets
-// of two: 100.1k as one set). So a tile costs about 250 clocks a level, 10 an
-// entry and 1.2 a wavefront, and wide tiles pay until the last round of tiles
-// leaves most SMs idle.
+// The cost of a tile-cycle in SM clocks was fitted to one wave of tiles on
+// netlists of 41 levels and 3,000 / 10,000 / 20,000 / 50,000 gates: one-word
+// rows 10.9k / 12.4k / 15.5k / 26.1k; one 4-word vector 12.9k / 17.4k / 22.7k
+// / 37.2k, two 16.4k / 24.8k / 33.5k / 56.1k, four as two warp sets of two
+// 24.8k / 36.9k / 53.9k / 97.8k (sets of one vector: four sets 25.3k / 37.1k
+// / 57.3k / 114k, two sets against two vectors 17.8k / 24.8k / 35.6k /
+// 62.5k). So a tile costs about 220 clocks a level and 9 an entry, and each
+// vector one a wavefront and 75 a level; wide tiles pay until the last round
+// of tiles leaves most SMs idle.
 constexpr FlatShape kFlatShapes[] = {{4, 2, 2}, {4, 3, 1}, {4, 2, 1}, {4, 1, 1}, {2, 1, 1}, {1, 1, 1}};
 // The tile width a flat run reports: several tiles of the widest documented
 // width that divides its own.
@@ -421,9 +424,10 @@ uint32_t flat_reported_words(uint32_t w) { return w == 16 ? 8 : w == 12 ? 4 : w;
 // Clocks of one tile-cycle, from the statistics of the program built for row
 // width `base`.
 double flat_tile_cost(const FlatProgram& fp, uint32_t base, const FlatShape& x) {
-  const double vec4 = (double)fp.wavefronts * (base == 4 ? 1.0 : base == 2 ? 1.85 : 3.4);  // wavefronts of 4-word rows
-  const double work = vec4 * (x.V == 4 ? 1.2 * x.N * x.Q : x.V == 2 ? 0.58 : 0.36);
-  return fp.n_levels * 250.0 + fp.n_entries * 10.0 + work + 600.0;
+  const double L = fp.n_levels, E = fp.n_entries;
+  if (x.V != 4) return 173.0 * L + (x.V == 2 ? 25.0 : 21.7) * E;
+  const double vec4 = (double)fp.wavefronts * (base == 4 ? 1.0 : base == 2 ? 1.9 : 3.6);  // wavefronts of 4-word rows
+  return 222.0 * L + 9.1 * E + x.N * x.Q * (1.03 * vec4 + 75.0 * L);
 }
 
 // The widest rows that fit (0: none); packing leaves fewer live nets than the

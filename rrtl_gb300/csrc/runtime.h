@@ -237,7 +237,7 @@ struct rrtl_design {
   // gate engine: one program per fused tile width W (index log2 W), built on
   // demand; nets, levels and registers are the same in every variant
   std::unique_ptr<rrtl::GateVariant> gvar[4];
-  std::unique_ptr<rrtl::FlatVariant> fvar[3][2][2];  // flat programs by log2 V, warp sets - 1, with a row for every signal
+  std::unique_ptr<rrtl::FlatVariant> fvar[3][3][2];  // flat programs by log2 V, log2 of the warp sets, with a row for every signal
   uint32_t gate_base = 3;   // log2 W of the variant built at load time
   uint32_t gate_w_max = 0;  // widest W whose slots fit on chip, 0 if none
   std::map<uint32_t, uint32_t> tuned_w;  // measured best W by lane bucket (ceil log2 of 32-lane words);

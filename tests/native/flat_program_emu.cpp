@@ -34,7 +34,7 @@ uint32_t two(uint32_t meta, uint32_t a, uint32_t b) {
 }  // namespace
 
 extern "C" int emu_flat_run(const char* json, size_t len, const char* top, uint32_t V, uint32_t pack, uint32_t fold,
-                            uint32_t warps, uint32_t max_slots, uint32_t lanes, uint64_t cycles, uint64_t seed,
+                            uint32_t max_warps, uint32_t max_slots, uint32_t lanes, uint64_t cycles, uint64_t seed,
                             uint64_t lane_base, uint32_t n_stim, const uint32_t* stim_sig, const uint32_t* stim_kind,
                             const uint64_t* stim_param, uint32_t n_rec, const uint32_t* rec_sig, uint64_t* out_hash,
                             uint32_t* stats, char* err, size_t errcap) {
@@ -46,13 +46,15 @@ extern "C" int emu_flat_run(const char* json, size_t len, const char* top, uint3
     opt.pack = pack != 0;
     opt.observe = pack == 2;  // 2: every signal keeps a row
     opt.fold_regs = fold != 0;
-    opt.warps = warps;
+    opt.max_warps = max_warps;
     opt.max_slots = max_slots;
     FlatProgram fp = build_flat_program(gp, V, opt);
     for (uint32_t s = 0; opt.observe && s < gp.n_signals; ++s) {
       const uint32_t net = gp.signal_net[s];
       if (!gp.net_is_source[net] && fp.net_slot[net] >= 0 && fp.net_level[net] < 0) throw Fail{"a row no cell writes"};
     }
+    const uint32_t warps = fp.warps;
+    if (warps < 1 || warps > max_warps) throw Fail{"streams"};
     if (stats) {
       const uint32_t s[] = {fp.n_two,   fp.n_three, fp.n_levels, fp.n_slots, fp.n_entries, (uint32_t)fp.wavefronts,
                             (uint32_t)fp.floor_wavefronts, (uint32_t)fp.commit.size()};
