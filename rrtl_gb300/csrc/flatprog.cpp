@@ -107,7 +107,7 @@ struct Logic {
   std::vector<uint8_t> root;     // net must be in its own row at the end of a cycle
   std::vector<uint32_t> commit;  // registers left on the commit list
   uint32_t n_levels = 0;
-  bool observe = false;
+  bool observe = false, settle = false;
 
   explicit Logic(const GateProgram& g) : gp(g) {}
 
@@ -149,7 +149,7 @@ struct Logic {
   void drop_dead() {
     std::vector<uint32_t> f = fanout();
     for (size_t i = cells.size(); i-- > 0;) {
-      if (!alive[i] || root[cells[i].out] || f[cells[i].out]) continue;
+      if (!alive[i] || root[cells[i].out] || f[cells[i].out] || (settle && gp.net_signal[cells[i].out] >= 0)) continue;
       alive[i] = 0;
       for (int k = 0; k < cells[i].n; ++k) --f[cells[i].in[k]];
     }
@@ -614,12 +614,13 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
   fp.V = V;
   const uint32_t G = fp.G = 32 / V;
   Logic lg(gp);
-  lg.observe = opt.observe;
+  lg.observe = opt.observe || opt.settle;
+  lg.settle = opt.settle;
   lg.collect();
   if (opt.pack) lg.pack();
   else lg.drop_dead();
   lg.levelize();
-  lg.fold_registers(opt.fold_regs);
+  lg.fold_registers(opt.fold_regs && !opt.settle);
   std::vector<FlatCell>& cells = lg.cells;
   const uint32_t NL = fp.n_levels = lg.n_levels;
   fp.commit = lg.commit;
@@ -637,11 +638,13 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
     else made[c.out] = c.level;
   }
   for (uint32_t r : lg.commit) {
+    q_write[gp.regs[r].q_net] = kEnd;
+    if (opt.settle) continue;  // no row is read after the levels
     last[gp.regs[r].d_net] = kEnd;
     if (gp.regs[r].has_reset) last[gp.regs[r].rst_net] = kEnd;
-    q_write[gp.regs[r].q_net] = kEnd;
   }
-  for (uint32_t n = 0; n < gp.n_nets; ++n)
+  if (opt.settle) fp.commit.clear();
+  for (uint32_t n = 0; n < gp.n_nets && !opt.settle; ++n)
     if (made[n] >= 0 && lg.root[n] && (gp.net_is_output[n] || last[n] >= kEnd)) last[n] = kEnd;
 
   // ---- residue balance: rows read per (level, residue)
@@ -764,6 +767,7 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
   struct Entry {
     std::vector<FlatLane> lanes;
     std::vector<uint32_t> outs;  // nets written
+    std::vector<uint32_t> nets;  // settle: signal net per lane and cell
     double cost = 0;
   };
   std::vector<std::vector<Entry>> entries(NL);
@@ -847,8 +851,14 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
       }
     };
     auto outs_of = [&](Entry& e, const std::vector<Group>& gs, size_t g0, size_t n) {
+      if (opt.settle) e.nets.assign(64, 0xFFFFFFFFu);
       for (size_t g = g0; g < std::min(gs.size(), g0 + n); ++g)
-        for (uint32_t ci : gs[g].cells) e.outs.push_back(cells[ci].out);
+        for (size_t k = 0; k < gs[g].cells.size(); ++k) {
+          const uint32_t net = cells[gs[g].cells[k]].out;
+          e.outs.push_back(net);
+          const size_t at_lane = g - g0;  // groups fill the lanes of the first cell, then those of the second
+          if (opt.settle && gp.net_signal[net] >= 0) e.nets[2 * (at_lane % V * G + k) + at_lane / V] = net;
+        }
     };
     for (size_t g = 0; g < g2.size(); g += 2 * V) {
       Entry e;
@@ -887,6 +897,7 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
   // 17.2k, 5 12.4k and 17.4k.
   const uint32_t warps = fp.warps = std::max(1u, std::min(opt.max_warps, NL ? (fp.n_entries + NL - 1) / NL : 1u));
   std::vector<std::vector<FlatLane>> streams(warps);
+  std::vector<std::vector<uint32_t>> stream_nets(warps);
   std::vector<uint32_t> last_level(warps, 0);
   for (uint32_t L = 0; L < NL; ++L) {
     std::vector<Entry>& es = entries[L];
@@ -913,6 +924,10 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
         if (syncs) l.y |= kFlatDevSync;
         streams[w].push_back(l);
       }
+      if (opt.settle) {
+        stream_nets[w].resize((streams[w].size() - 32) * 2, 0xFFFFFFFFu);
+        stream_nets[w].insert(stream_nets[w].end(), e.nets.begin(), e.nets.end());
+      }
     }
   }
   if (next_slot > kMaxSlots) next_slot = kMaxSlots + 1;
@@ -924,6 +939,10 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
     fp.warp_tail[w] = NL ? NL - 1 - last_level[w] : 0;
     fp.warp_begin[w + 1] = fp.warp_begin[w] + (uint32_t)(streams[w].size() / 32);
     fp.stream.insert(fp.stream.end(), streams[w].begin(), streams[w].end());
+    if (opt.settle) {
+      stream_nets[w].resize(streams[w].size() * 2, 0xFFFFFFFFu);
+      fp.stream_net.insert(fp.stream_net.end(), stream_nets[w].begin(), stream_nets[w].end());
+    }
   }
   fp.recordable.assign(gp.n_nets, 0);
   for (uint32_t n = 2; n < gp.n_nets; ++n) {

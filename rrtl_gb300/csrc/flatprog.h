@@ -70,6 +70,7 @@ struct FlatProgram {
   std::vector<uint32_t> source_nets;      // loaded at the start of a run, written back at its end
   std::vector<uint32_t> commit;           // GateProgram::regs indices not folded
   std::vector<FlatLane> stream;           // [entry][32 lanes]
+  std::vector<uint32_t> stream_net;       // settle: [entry][32][2] signal net each cell writes back, ~0: none
   std::vector<uint32_t> warp_begin;       // per warp: first entry (a multiple of kFlatPrefetch); size warps + 1
   std::vector<uint32_t> warp_tail;        // level barriers after a warp's last entry
   // shared-memory wavefronts of one row vector's cell accesses, and their floor
@@ -80,6 +81,7 @@ struct FlatProgram {
 struct FlatOptions {
   bool pack = true;
   bool fold_regs = true;
+  bool settle = false;   // a closing settle: every signal computed and written back, no registers committed
   bool observe = false;  // every signal keeps a row of its own (stuck-at forces act on any of them)
   uint32_t max_warps = kFlatComputeThreads / 32;  // of the set; a program of few entries a level uses fewer
   uint32_t max_slots = 0;  // above this, a row is placed at any residue before the slot array grows (0: no limit)

@@ -92,6 +92,7 @@ struct GateProgDev {
 // A flat gate program on the device (flatprog.h).
 struct FlatProgDev {
   const uint4* stream;         // [entry][32] FlatLane
+  const uint2* stream_net;     // closing settle: [entry][32] signal nets the entry's cells write back, ~0: none
   const uint32_t* warp_begin;  // [warps + 1]
   const uint32_t* warp_tail;   // [warps]
   const uint32_t* src_net;
@@ -155,7 +156,8 @@ struct GateItemDev {
 struct FlatJobDev {
   FlatProgDev P;
   GateRunDev R;
-  uint32_t shape, pad;  // V * 100 + N * 10 + Q
+  uint32_t shape;   // V * 100 + N * 10 + Q
+  uint32_t settle;  // a closing settle (flat_settle_tile)
 };
 
 struct FlatQueueDev {

@@ -41,11 +41,40 @@ cudaError_t launch_gate_flat(uint32_t V, uint32_t N, uint32_t Q, const FlatProgD
   }
 }
 
+template <int V, int N>
+__global__ void __launch_bounds__(kFlatThreads, 1) gate_flat_settle_kernel(FlatProgDev P, GateRunDev R) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  for (uint32_t tile = blockIdx.x; tile < R.n_tiles; tile += gridDim.x) flat_settle_tile<V, N>(P, R, tile, smem);
+}
+
+template <int V, int N>
+static cudaError_t launch_settle(const FlatProgDev& P, const GateRunDev& R, uint32_t grid, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(gate_flat_settle_kernel<V, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlatSmem);
+  if (e != cudaSuccess) return e;
+  gate_flat_settle_kernel<V, N><<<grid, kFlatThreads, kFlatSmem, st>>>(P, R);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_gate_flat_settle(uint32_t V, uint32_t N, const FlatProgDev& P, const GateRunDev& R, uint32_t grid,
+                                    cudaStream_t st) {
+  switch (V * 10 + N) {
+    case 42: return launch_settle<4, 2>(P, R, grid, st);
+    case 41: return launch_settle<4, 1>(P, R, grid, st);
+    case 21: return launch_settle<2, 1>(P, R, grid, st);
+    case 11: return launch_settle<1, 1>(P, R, grid, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 // Persistent queue kernel: CTAs take (job, tile) items, all cycles of the
 // job, from a device list (longest first) until it is empty. The job's
 // descriptor lies in the header of shared memory, behind the detection state.
 template <int V, int N, int Q>
 __device__ __forceinline__ void queue_tile(const FlatJobDev& J, const GateItemDev& item, uint8_t* smem) {
+  if (J.settle) {
+    if constexpr (Q == 1) flat_settle_tile<V, N>(J.P, J.R, item.tile, smem);
+    return;
+  }
   if (J.R.has_forces) flat_tile<V, N, Q, true, false>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
   else flat_tile<V, N, Q, false, false>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
 }

@@ -166,8 +166,9 @@ __device__ __forceinline__ const typename FlatVec<V>::T* flat_row(const uint8_t*
 // other's rows, so every load of an entry may precede its stores (which the
 // compiler cannot know). Functions and row addresses are decoded before the
 // level barrier the entry may wait for.
-template <int V, int N, int Q, class Bar>
-__device__ __forceinline__ void flat_pair2(uint8_t* S, const uint4& r, uint32_t go, const Bar& bar) {
+// `out` sees every row vector written: out(which cell, plane, value).
+template <int V, int N, int Q, class Bar, class Out>
+__device__ __forceinline__ void flat_pair2(uint8_t* S, const uint4& r, uint32_t go, const Bar& bar, const Out& out) {
   using T = typename FlatVec<V>::T;
   constexpr uint32_t kStep = flat_plane_bytes(N * Q) / sizeof(T);
   constexpr int H = N > 2 ? 2 : N;  // planes whose operands are in registers at once
@@ -193,14 +194,17 @@ __device__ __forceinline__ void flat_pair2(uint8_t* S, const uint4& r, uint32_t 
 #pragma unroll
     for (int p = 0; p < H; ++p) {
       if (p0 + p >= N) break;
-      po[(p0 + p) * kStep] = f(a[p], b[p]);
-      pq[(p0 + p) * kStep] = g(c[p], d[p]);
+      const T v = f(a[p], b[p]), w = g(c[p], d[p]);
+      po[(p0 + p) * kStep] = v;
+      pq[(p0 + p) * kStep] = w;
+      out(0, p0 + p, v);
+      out(1, p0 + p, w);
     }
   }
 }
 
-template <int V, int N, int Q, class Bar>
-__device__ __forceinline__ void flat_one3(uint8_t* S, const uint4& r, uint32_t go, const Bar& bar) {
+template <int V, int N, int Q, class Bar, class Out>
+__device__ __forceinline__ void flat_one3(uint8_t* S, const uint4& r, uint32_t go, const Bar& bar, const Out& out) {
   using T = typename FlatVec<V>::T;
   constexpr uint32_t kStep = flat_plane_bytes(N * Q) / sizeof(T);
   constexpr int H = N > 2 ? 2 : N;
@@ -223,10 +227,17 @@ __device__ __forceinline__ void flat_one3(uint8_t* S, const uint4& r, uint32_t g
 #pragma unroll
     for (int p = 0; p < H; ++p) {
       if (p0 + p >= N) break;
-      po[(p0 + p) * kStep] = f(a[p], b[p], c[p]);
+      const T v = f(a[p], b[p], c[p]);
+      po[(p0 + p) * kStep] = v;
+      out(0, p0 + p, v);
     }
   }
 }
+
+struct FlatNoOut {
+  template <class T>
+  __device__ __forceinline__ void operator()(int, int, const T&) const {}
+};
 
 // Stuck-at forces of the comb nets one warp writes, applied by that warp when
 // it finished a level, before the level's barrier: no barrier of their own.
@@ -275,6 +286,77 @@ __device__ __forceinline__ void flat_bar_compute() {
   asm volatile("bar.sync 6, %0;" ::"n"(kFlatComputeThreads) : "memory");
 }
 
+// Source rows of a tile of W words in (words past the padded batch read as zero).
+template <int V, uint32_t W, uint32_t kPlane>
+__device__ __forceinline__ void flat_load_sources(const FlatProgDev& P, const GateRunDev& R, uint32_t col0, uint8_t* S) {
+  for (uint32_t i = threadIdx.x; i < P.n_src * W; i += blockDim.x) {
+    const uint32_t k = i / W, ww = i % W;
+    *reinterpret_cast<uint32_t*>(S + (ww / V) * kPlane + __ldg(P.src_slot + k) * (V * 4u) + (ww % V) * 4u) =
+        col0 + ww < R.words_pad ? R.nets[(size_t)__ldg(P.src_net + k) * R.words_pad + col0 + ww] : 0u;
+  }
+}
+
+// Closing settle of one tile (V * N words): the levels once, every signal net
+// written back to the run's global rows as it is computed. Bound: the
+// write-back (4 bytes a signal and word) and, in small batches, the level
+// chain. As a separate fused-kernel launch at its widest tile the settle left
+// most SMs idle in small batches and stored word by word: whole runs that end
+// with this one instead went from 1.51 to 1.41 ms (50,000 gates, 200 lanes,
+// 100 cycles), 3.26 to 3.11 (5,003 lanes, 200 cycles), 7.04 to 6.35 (200,000
+// gates, 10,007 lanes, 100 cycles) and 47.5 to 47.2 (65,536 lanes, 1,000).
+template <int V, int N>
+__device__ __forceinline__ void flat_settle_tile(const FlatProgDev& P, const GateRunDev& R, uint32_t tile, uint8_t* smem) {
+  using T = typename FlatVec<V>::T;
+  constexpr uint32_t W = V * N;
+  constexpr int D = (int)kFlatPrefetch;
+  uint8_t* const S = smem + kFlatHeader;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, col0 = tile * W;
+  flat_load_sources<V, W, flat_plane_bytes(N)>(P, R, col0, S);
+  __syncthreads();
+  if (warp < P.warps) {
+    const FlatBar<0> bar{2u, P.warps * 32u};
+    const uint32_t begin = __ldg(P.warp_begin + warp), n = __ldg(P.warp_begin + warp + 1) - begin;
+    const uint4* const base = P.stream + (size_t)begin * 32u + lane;
+    const uint2* const nets = P.stream_net + (size_t)begin * 32u + lane;
+    uint4 q[D];
+    uint2 w[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      q[d] = n ? flat_load_entry(base + d * 32) : make_uint4(0u, 0u, 0u, 0u);
+      w[d] = n ? __ldg(nets + d * 32) : make_uint2(0u, 0u);
+    }
+    for (uint32_t e = 0; e < n; e += D) {
+      const uint32_t ahead = e + D < n ? e + D : 0u;
+      uint4 nx[D];
+      uint2 wx[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        nx[d] = flat_load_entry(base + (size_t)(ahead + d) * 32u);
+        wx[d] = __ldg(nets + (size_t)(ahead + d) * 32u);
+      }
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const uint4 r = q[d];
+        const uint2 id = w[d];
+        auto out = [&](int h, int plane, const T& v) {
+          const uint32_t net = h ? id.y : id.x, col = col0 + (uint32_t)plane * V;
+          if (net != 0xFFFFFFFFu && col < R.words_pad) *reinterpret_cast<T*>(R.nets + (size_t)net * R.words_pad + col) = v;
+        };
+        const uint32_t go = r.y & kFlatDevSync;
+        if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, 1>(S, r, go, bar, out);
+        else flat_pair2<V, N, 1>(S, r, go, bar, out);
+      }
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        q[d] = nx[d];
+        w[d] = wx[d];
+      }
+    }
+    for (uint32_t k = __ldg(P.warp_tail + warp); k; --k) bar.pass(1u);
+  }
+  __syncthreads();
+}
+
 // Cycles [c0, c0 + ncyc) of one tile (V * N * Q words) of a run; F: with
 // stuck-at forces; kFull: the program has a stream for every warp of a set.
 // Source nets are read from and written back to the run's global rows; the
@@ -292,12 +374,7 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
   auto word_at = [&](uint32_t slot, uint32_t ww) -> uint32_t& {  // word ww of the tile
     return *reinterpret_cast<uint32_t*>(S + (ww / V) * kPlane + slot * (V * 4u) + (ww % V) * 4u);
   };
-  // sources in (words past the padded batch read as zero)
-  for (uint32_t i = tid; i < P.n_src * W; i += blockDim.x) {
-    const uint32_t k = i / W, ww = i % W;
-    word_at(__ldg(P.src_slot + k), ww) =
-        col0 + ww < R.words_pad ? R.nets[(size_t)__ldg(P.src_net + k) * R.words_pad + col0 + ww] : 0u;
-  }
+  flat_load_sources<V, W, kPlane>(P, R, col0, S);
   if (tid < 16u) {
     // lanes already detected by an earlier part of this run stay detected
     uint32_t det = 0u;
@@ -350,8 +427,8 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
             if (go) forces.apply(S, level, lane);  // the same on every lane
           }
           // (the vote makes the branch a warp-uniform one)
-          if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, Q>(Sq, r, go, bar);
-          else flat_pair2<V, N, Q>(Sq, r, go, bar);
+          if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, Q>(Sq, r, go, bar, FlatNoOut{});
+          else flat_pair2<V, N, Q>(Sq, r, go, bar, FlatNoOut{});
           if constexpr (F) {
             if (go) forces.advance(level++);
           }
@@ -393,7 +470,7 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
     }
   } else {
     const uint32_t st = tid - kFlatComputeThreads;
-    constexpr int KS = 8, KR = 8;  // stimulus and record words a thread holds in registers
+    constexpr int KS = 10, KR = 8;  // stimulus and record words a thread holds in registers
     const uint32_t n_stim = R.n_stim * W, n_rec = R.n_rec * W;
     uint32_t sv[KS], rv[KR];
     auto stim_of = [&](uint32_t i, uint64_t c) -> uint32_t {  // never HOLD

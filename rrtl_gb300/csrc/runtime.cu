@@ -23,6 +23,8 @@ int gate_fused_ctas_per_sm(const GateProgDev& P, size_t smem);
 cudaError_t launch_gate_fused(const GateProgDev& P, const GateRunDev& R, uint32_t grid, size_t smem, cudaStream_t st);
 cudaError_t launch_gate_flat(uint32_t V, uint32_t N, uint32_t Q, const FlatProgDev& P, const GateRunDev& R, uint32_t grid,
                              cudaStream_t st);
+cudaError_t launch_gate_flat_settle(uint32_t V, uint32_t N, const FlatProgDev& P, const GateRunDev& R, uint32_t grid,
+                                    cudaStream_t st);
 cudaError_t launch_gate_flat_queue(const FlatQueueDev& L, uint32_t grid, cudaStream_t st);
 cudaError_t launch_gate_plain(const GateProgDev& P, const GateRunDev& R, uint64_t c, int phase, cudaStream_t st);
 cudaError_t launch_word(const WordProgDev& P, const WordRunDev& R, bool smem_slots, cudaStream_t st);
@@ -278,10 +280,11 @@ GateVariant* gate_variant(rrtl_design* d, uint32_t W) {
 }
 
 // Build and upload the flat program of row width V for Q warp sets; observe:
-// with a row for every signal (runs with stuck-at forces).
-FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe) {
+// with a row for every signal (runs with stuck-at forces); settle: the closing settle's.
+FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe, bool settle = false) {
   std::lock_guard<std::mutex> lk(d->gvar_mu);
-  std::unique_ptr<FlatVariant>& slot = d->fvar[log2_words(V)][log2_words(Q)][observe ? 1 : 0];
+  std::unique_ptr<FlatVariant>& slot =
+      settle ? d->fvar_settle[log2_words(V)] : d->fvar[log2_words(V)][log2_words(Q)][observe ? 1 : 0];
   if (slot) return slot.get();
   auto v = std::make_unique<FlatVariant>();
   const GateProgram& gp = d->gp();
@@ -295,6 +298,7 @@ FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe) 
   FlatOptions o;
   o.max_warps = kFlatComputeThreads / 32 / Q;
   o.observe = observe;
+  o.settle = settle;
   v->fp = build_flat_program(gp, V, o);
   v->max_n = fit(v->fp.n_slots);
   if (v->max_n < top) {
@@ -323,12 +327,14 @@ FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe) 
       commit.push_back(GateRegDev{row(r.q_net), row(r.d_net), r.has_reset ? row(r.rst_net) : kFlatConst0, fl});
     }
     upload(v->d_stream, fp.stream);
+    upload(v->d_stream_net, fp.stream_net);
     upload(v->d_warps, warps);
     upload(v->d_src_net, fp.source_nets);
     upload(v->d_src_slot, src_slot);
     upload(v->d_commit, commit);
     FlatProgDev& P = v->dev;
     P.stream = v->d_stream.as<uint4>();
+    P.stream_net = v->d_stream_net.as<uint2>();
     P.warp_begin = v->d_warps.as<uint32_t>();
     P.warp_tail = P.warp_begin + fp.warps + 1;
     P.src_net = v->d_src_net.as<uint32_t>();
@@ -475,6 +481,29 @@ FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w, uint3
     }
   }
   return checked(s);
+}
+
+// Shape of a closing settle over `words` words (V = 0: none fits), by the cost
+// of one tile-cycle of the cycles' program: its settle has the unpacked cells
+// (1.3 times the entries), the same for every shape.
+FlatShape choose_settle(rrtl_design* d, uint32_t words) {
+  FlatShape s;
+  uint32_t top = 0;
+  for (uint32_t V = 4; V >= 1 && !top; V /= 2)
+    if ((size_t)d->gp().n_slots * V * 4 <= flat_plane_bytes(1) / 4 * 5 && flat_variant(d, V, 1, false, true)->max_n) top = V;
+  if (!top) return s;
+  const FlatVariant* v = flat_variant(d, top, 1, false, true);
+  double best = INFINITY;
+  for (const FlatShape& x : {FlatShape{4, 2, 1}, FlatShape{4, 1, 1}, FlatShape{2, 1, 1}, FlatShape{1, 1, 1}}) {
+    if (x.V > top || (x.V == 4 && x.N > v->max_n)) continue;
+    const double t = std::ceil(std::ceil((double)words / x.words()) / d->ctx->sm_count) * flat_tile_cost(v->fp, top, x);
+    if (t < best) {
+      best = t;
+      s = x;
+    }
+  }
+  if (s.V && flat_variant(d, s.V, 1, false, true)->max_n < s.N) s.V = 0;
+  return s;
 }
 
 void upload_word_program(rrtl_design* d) {
@@ -672,6 +701,10 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   if (flat.V) {
     g.flat = flat_variant(d, flat.V, flat.Q, !b->faults.empty());
     g.shape = flat;
+    // the fused kernel's settle applies stuck-at forces; without them the flat
+    // one is faster at every size tried (200 to 65,536 lanes, 50k and 200k gates)
+    if (b->faults.empty()) g.settle_shape = choose_settle(d, b->words);
+    if (g.settle_shape.V) g.settle = flat_variant(d, g.settle_shape.V, 1, false, true);
   }
   // (the fused kernel only closes a flat run: the variant built at load time does)
   const uint32_t W = !want_fused ? 0
@@ -811,16 +844,22 @@ GateRunDev closing_desc(const GatePrepared& g) {
   C.n_stim = 0;
   C.n_rec = 0;
   C.mode = 0;
-  C.n_tiles = g.R.words_pad / g.W;
+  C.n_tiles = g.settle ? (g.R.words_pad + g.settle_shape.words() - 1) / g.settle_shape.words() : g.R.words_pad / g.W;
   return C;
 }
 
-// A flat run: the cycles on the flat kernel, then the closing settle, which
-// writes every signal back, on the fused kernel.
+// A flat run: the cycles, then the closing settle, which writes every signal
+// back (with stuck-at forces on the fused kernel).
 void gate_flat_launch(rrtl_design* d, const GatePrepared& g, cudaStream_t st) {
   const GateRunDev R = flat_run_desc(g), C = closing_desc(g);
   cuda_check(launch_gate_flat(g.shape.V, g.shape.N, g.shape.Q, g.flat->dev, R, std::min(R.n_tiles, d->ctx->sm_count), st),
              "gate_flat_kernel");
+  if (g.settle) {
+    cuda_check(launch_gate_flat_settle(g.settle_shape.V, g.settle_shape.N, g.settle->dev, C,
+                                       std::min(C.n_tiles, d->ctx->sm_count), st),
+               "gate_flat_settle_kernel");
+    return;
+  }
   const uint32_t grid = std::min<uint32_t>(C.n_tiles, d->ctx->sm_count * g.v->fused_ctas);
   cuda_check(launch_gate_fused(g.v->gdev, C, grid, g.v->fused_smem, st), "gate_fused_kernel");
 }
@@ -1356,8 +1395,9 @@ std::vector<FlatShape> queue_shapes(rrtl_ctx* c, const std::vector<QueueJob*>& j
 
 // One persistent launch over every queued job: each job's tiles become items
 // (all cycles of one tile), listed longest first. Jobs the flat kernel takes
-// run there and leave their closing settle to the fused queue kernel behind
-// it, which also runs the other jobs; jobs whose recorded nets leave the chip,
+// run there, their closing settles in a second launch of it; the fused queue
+// kernel behind them runs the other jobs and the closing settles of fault
+// jobs; jobs whose recorded nets leave the chip,
 // or whose shared memory exceeds what the queue kernel can take, run on their
 // own kernels first on the same stream.
 void queue_launch(rrtl_ctx* c) {
@@ -1367,7 +1407,7 @@ void queue_launch(rrtl_ctx* c) {
   std::vector<GateJobDev> jobs;
   std::vector<FlatJobDev> flat_jobs;
   using Item = std::pair<double, GateItemDev>;
-  std::vector<Item> items, flat_items;
+  std::vector<Item> items, flat_items, settle_items;
   size_t smem = 0;
   const uint32_t launch = ++Q.launches;
   std::vector<QueueJob*> todo;
@@ -1395,15 +1435,23 @@ void queue_launch(rrtl_ctx* c) {
       continue;
     }
     const uint32_t ji = (uint32_t)jobs.size();
-    smem = std::max(smem, g.v->fused_smem);
+    if (!g.settle) smem = std::max(smem, g.v->fused_smem);
     if (g.flat) {
       const GateRunDev R = flat_run_desc(g);
       const double cost = (double)j.run.cycles * flat_tile_cost(g.flat->fp, g.shape.V, g.shape);
       for (uint32_t t = 0; t < R.n_tiles; ++t)
         flat_items.push_back({cost, GateItemDev{(uint32_t)flat_jobs.size(), t, 0ull, (uint32_t)j.run.cycles, 0u}});
       flat_jobs.push_back(FlatJobDev{g.flat->dev, R, g.shape.V * 100 + g.shape.N * 10 + g.shape.Q, 0u});
-      jobs.push_back(GateJobDev{g.v->gdev, closing_desc(g)});
       b->last_tile_words = flat_reported_words(g.shape.words());
+      if (g.settle) {
+        const GateRunDev C = closing_desc(g);
+        const double c = flat_tile_cost(g.settle->fp, g.settle_shape.V, g.settle_shape);
+        for (uint32_t t = 0; t < C.n_tiles; ++t)
+          settle_items.push_back({c, GateItemDev{(uint32_t)flat_jobs.size(), t, 0ull, 0u, 0u}});
+        flat_jobs.push_back(FlatJobDev{g.settle->dev, C, g.settle_shape.V * 100 + g.settle_shape.N * 10 + 1, 1u});
+        continue;
+      }
+      jobs.push_back(GateJobDev{g.v->gdev, closing_desc(g)});
     } else {
       jobs.push_back(GateJobDev{g.v->gdev, g.R});
       b->last_tile_words = g.W;
@@ -1413,7 +1461,7 @@ void queue_launch(rrtl_ctx* c) {
     for (uint32_t t = 0; t < jobs.back().R.n_tiles; ++t)
       items.push_back({cost, GateItemDev{ji, t, 0ull, (uint32_t)cycles, 1u}});
   }
-  Q.last_items = (uint32_t)(items.size() + flat_items.size());
+  Q.last_items = (uint32_t)(items.size() + flat_items.size() + settle_items.size());
   auto stage = [&](std::vector<Item>& v, DevBuf& d) {
     std::stable_sort(v.begin(), v.end(), [](const Item& x, const Item& y) { return x.first > y.first; });
     std::vector<GateItemDev> flat;
@@ -1421,18 +1469,24 @@ void queue_launch(rrtl_ctx* c) {
     for (auto& it : v) flat.push_back(it.second);
     upload(d, flat);
   };
+  if (!items.empty() || !flat_items.empty()) {
+    Q.d_next.reserve(16);
+    cuda_check(cudaMemsetAsync(Q.d_next.p, 0, 16, st), "memset queue");
+  }
+  if (!flat_items.empty()) {
+    upload(Q.d_flat_jobs, flat_jobs);
+    auto run = [&](std::vector<Item>& v, DevBuf& d, uint32_t counter) {
+      if (v.empty()) return;
+      stage(v, d);
+      FlatQueueDev L{Q.d_flat_jobs.as<FlatJobDev>(), d.as<GateItemDev>(), (uint32_t)v.size(), Q.d_next.as<uint32_t>() + counter};
+      cuda_check(launch_gate_flat_queue(L, std::min<uint32_t>(L.n_items, c->sm_count), st), "gate_flat_queue_kernel");
+    };
+    run(flat_items, Q.d_flat_items, 2);
+    run(settle_items, Q.d_settle_items, 3);
+  }
   if (!items.empty()) {
     stage(items, Q.d_items);
     upload(Q.d_jobs, jobs);
-    Q.d_next.reserve(16);
-    cuda_check(cudaMemsetAsync(Q.d_next.p, 0, 16, st), "memset queue");
-    if (!flat_items.empty()) {
-      stage(flat_items, Q.d_flat_items);
-      upload(Q.d_flat_jobs, flat_jobs);
-      FlatQueueDev L{Q.d_flat_jobs.as<FlatJobDev>(), Q.d_flat_items.as<GateItemDev>(), (uint32_t)flat_items.size(),
-                     Q.d_next.as<uint32_t>() + 2};
-      cuda_check(launch_gate_flat_queue(L, std::min<uint32_t>(L.n_items, c->sm_count), st), "gate_flat_queue_kernel");
-    }
     if (!Q.smem_set) {
       // the limit is per kernel: allow every job this queue can take
       cuda_check(gate_queue_prepare(qmax), "gate_queue_prepare");

@@ -73,7 +73,7 @@ struct FlatVariant {
   FlatProgram fp;
   FlatProgDev dev{};
   uint32_t max_n = 0;  // vectors of V words that fit in shared memory, 0: none
-  DevBuf d_stream, d_warps, d_src_net, d_src_slot, d_commit;
+  DevBuf d_stream, d_stream_net, d_warps, d_src_net, d_src_slot, d_commit;
 };
 
 // A shape of the flat kernel: row width V (0: none), vectors per warp set N,
@@ -107,6 +107,9 @@ struct GatePrepared {
   // the flat kernel runs the cycles and the fused kernel the closing settle
   FlatVariant* flat = nullptr;
   FlatShape shape;
+  // flat form of the closing settle (nullptr: the fused kernel's)
+  FlatVariant* settle = nullptr;
+  FlatShape settle_shape;
   size_t trace_out_bytes = 0, hash_bytes = 0, det_bytes = 0;
   bool want_trace = false, want_hash = false, want_det = false;
 };
@@ -139,7 +142,7 @@ struct JobQueue {
   uint32_t launches = 0;
   std::vector<QueueJob> jobs;                 // queued or running
   std::unordered_map<uint64_t, uint32_t> finished;  // id -> RRTL_JOB_DONE / RRTL_JOB_FAILED
-  DevBuf d_jobs, d_items, d_next, d_flat_jobs, d_flat_items;
+  DevBuf d_jobs, d_items, d_next, d_flat_jobs, d_flat_items, d_settle_items;
   size_t smem_set = 0;                        // dynamic shared memory the queue kernel is prepared for
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;   // around the last launch
   float last_ms = 0.f;
@@ -238,6 +241,7 @@ struct rrtl_design {
   // demand; nets, levels and registers are the same in every variant
   std::unique_ptr<rrtl::GateVariant> gvar[4];
   std::unique_ptr<rrtl::FlatVariant> fvar[3][3][2];  // flat programs by log2 V, log2 of the warp sets, with a row for every signal
+  std::unique_ptr<rrtl::FlatVariant> fvar_settle[3];  // closing settles by log2 V
   uint32_t gate_base = 3;   // log2 W of the variant built at load time
   uint32_t gate_w_max = 0;  // widest W whose slots fit on chip, 0 if none
   std::map<uint32_t, uint32_t> tuned_w;  // measured best W by lane bucket (ceil log2 of 32-lane words);

@@ -8,6 +8,7 @@
 // the per-cycle output hash follow stim.h.
 #include <cstdint>
 #include <cstdio>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -45,6 +46,7 @@ extern "C" int emu_flat_run(const char* json, size_t len, const char* top, uint3
     FlatOptions opt;
     opt.pack = pack != 0;
     opt.observe = pack == 2;  // 2: every signal keeps a row
+    opt.settle = pack == 3;   // 3: the closing settle's program, its signal nets taken from its write-back
     opt.fold_regs = fold != 0;
     opt.max_warps = max_warps;
     opt.max_slots = max_slots;
@@ -71,14 +73,28 @@ extern "C" int emu_flat_run(const char* json, size_t len, const char* top, uint3
     std::vector<uint32_t> rec_net(n_rec), stim_net(n_stim);
     for (uint32_t i = 0; i < n_rec; ++i) {
       rec_net[i] = gp.signal_net.at(rec_sig[i]);
-      if (!fp.recordable[rec_net[i]]) fail("a recorded net is not recordable");
+      if (!opt.settle && !fp.recordable[rec_net[i]]) fail("a recorded net is not recordable");
     }
     for (uint32_t i = 0; i < n_stim; ++i) stim_net[i] = gp.signal_net.at(stim_sig[i]);
     if (fp.warp_begin.size() != warps + 1) fail("warp table size");
     for (uint32_t w = 0; w < warps; ++w)
       if ((fp.warp_begin[w + 1] - fp.warp_begin[w]) % kFlatPrefetch) fail("a stream is not a multiple of the prefetch");
+    if (fp.stream_net.size() != (opt.settle ? fp.stream.size() * 2 : 0)) fail("write-back table size");
+    if (opt.settle && !fp.commit.empty()) fail("a settle commits registers");
+    std::vector<std::vector<uint32_t>> back(opt.settle ? gp.n_nets : 0);
+    std::map<std::pair<uint32_t, uint32_t>, uint32_t> row_net;  // level and row written -> net
+    for (uint32_t n = 0; opt.settle && n < gp.n_nets; ++n)
+      if (!gp.net_is_source[n] && fp.net_level[n] >= 0) row_net[{(uint32_t)fp.net_level[n], (uint32_t)fp.net_slot[n]}] = n;
+    auto value = [&](uint32_t net) -> const uint32_t* {  // a net's words at the end of the cycle
+      if (!opt.settle || gp.net_is_source[net]) return row((uint32_t)fp.net_slot[net]);
+      if (back[net].empty()) throw Fail{"a net that is not written back"};
+      return back[net].data();
+    };
+    std::vector<uint32_t> commit = fp.commit;
+    for (uint32_t k = 0; opt.settle && k < gp.regs.size(); ++k) commit.push_back(k);
     std::vector<uint64_t> wrote(fp.n_slots, ~0ull), read(fp.n_slots, ~0ull);  // lane that touched the row in this level
     for (uint64_t c = 0; c < cycles; ++c) {
+      for (auto& v : back) v.clear();
       for (uint32_t i = 0; i < n_stim; ++i)
         for (uint32_t w = 0; w < words; ++w) {
           uint32_t& v = row((uint32_t)fp.net_slot[stim_net[i]])[w];
@@ -135,6 +151,14 @@ extern "C" int emu_flat_run(const char* json, size_t len, const char* top, uint3
                   }
                 }
                 for (uint32_t q = 0; q < words; ++q) row(so)[q] = out[q];
+                const uint32_t net = opt.settle ? fp.stream_net[((size_t)at[w] * 32 + l) * 2 + (uint32_t)h] : ~0u;
+                if (opt.settle && so >= fp.G) {
+                  const uint32_t made = row_net.at({L, so});
+                  if (net != (gp.net_signal[made] >= 0 ? made : ~0u)) fail("a write-back of another net");
+                  back[made] = out;
+                } else if (net != ~0u) {
+                  fail("an idle lane writes back");
+                }
               }
             }
           }
@@ -147,16 +171,18 @@ extern "C" int emu_flat_run(const char* json, size_t len, const char* top, uint3
       for (uint32_t k = 0; k < n_rec; ++k)
         for (uint32_t w = 0; w < words; ++w) {
           const uint32_t left = lanes - w * 32, vm = left >= 32 ? 0xFFFFFFFFu : (1u << left) - 1u;
-          hs += hash_term(c, k, word_base + w, row((uint32_t)fp.net_slot[rec_net[k]])[w] & vm);
+          hs += hash_term(c, k, word_base + w, value(rec_net[k])[w] & vm);
         }
       out_hash[c] = hs;
-      for (uint32_t k : fp.commit) {
+      for (uint32_t s = 0; opt.settle && s < gp.n_signals; ++s)
+        if (gp.signal_net[s] > kNetConst1) value(gp.signal_net[s]);
+      for (uint32_t k : commit) {
         const GateReg& r = gp.regs[k];
         for (uint32_t w = 0; w < words; ++w) {
-          uint32_t v = r.d_net == kNetConst0 ? 0u : r.d_net == kNetConst1 ? 0xFFFFFFFFu : row((uint32_t)fp.net_slot[r.d_net])[w];
+          uint32_t v = r.d_net == kNetConst0 ? 0u : r.d_net == kNetConst1 ? 0xFFFFFFFFu : value(r.d_net)[w];
           if (r.has_reset) {
             uint32_t m = r.rst_net == kNetConst0 ? 0u : r.rst_net == kNetConst1 ? 0xFFFFFFFFu
-                                                                               : row((uint32_t)fp.net_slot[r.rst_net])[w];
+                                                                               : value(r.rst_net)[w];
             if (r.active_low) m = ~m;
             v = r.reset_value ? v | m : v & ~m;
           }

@@ -82,6 +82,23 @@ def test_netlist_equals_the_oracle(emu, netlist, V, warps, pack, fold):
     assert st["floor"] <= st["wavefronts"] <= 1.10 * st["floor"], st
 
 
+@pytest.mark.parametrize("V", [4, 2, 1])
+def test_closing_settle_writes_every_signal_back(emu, netlist, V):
+    """The settle's program alone, its write-backs and the source rows standing for every net."""
+    js, meta, od = netlist
+    stim, rec = netlist_run_spec(meta)
+    rec = list(dict.fromkeys(rec + meta.gate_names))
+    h, st = _emulate(emu, js, meta.top, od, stim, rec, 40, 6, 17, V, pack=3)
+    assert np.array_equal(h, _oracle(od, stim, rec, 40, 6, 17))
+    d, top, outs = _register_mix()
+    js = d.to_json()
+    od = ob.OracleDesign(js, top)
+    stim = [("clk", sim.STIM_CONST, 1), ("rst", sim.STIM_PULSE, 3), ("rstn", sim.STIM_RANDOM, 9),
+            ("a", sim.STIM_RANDOM, 1), ("b", sim.STIM_RANDOM, 2), ("c", sim.STIM_RANDOM, 3)]
+    h, _ = _emulate(emu, js, top, od, stim, outs, 70, 20, 13, V, pack=3)
+    assert np.array_equal(h, _oracle(od, stim, outs, 70, 20, 13))
+
+
 def test_a_shorter_slot_array_keeps_the_results(emu, netlist):
     js, meta, od = netlist
     stim, rec = netlist_run_spec(meta)

@@ -172,3 +172,18 @@ def test_queue_of_flat_and_fused_jobs(wide, monkeypatch):
         for k in ("trace", "hash", "detect"):
             assert (a[k] is None and b[k] is None) or np.array_equal(a[k], b[k]), k
         assert np.array_equal(sa, sb)
+
+
+@pytest.mark.parametrize("lanes", [33, 32 * 16 * 3 + 7, 32 * 2500])
+def test_closing_settle_writes_every_signal(wide, monkeypatch, lanes):
+    """Lanes for its widths of 1, 4 and 8 words: each signal as the fused kernel leaves it."""
+    cd, meta, od = wide
+    stim, rec = netlist_run_spec(meta)
+    got = []
+    for flat in ("411", "0"):
+        monkeypatch.setenv("RRTL_FLAT", flat)
+        g = sim.GpuBatchSimulator(cd, lanes=lanes)
+        g.run(5, seed=4, stim=stim, record=rec, mode=sim.REC_HASH)
+        step = 1 if lanes < 5000 else 41
+        got.append([g.get_signal_bits(n) for n in (meta.inputs + meta.regs + meta.gate_names)[::step]])
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
