@@ -24,10 +24,38 @@ constexpr uint32_t kFlatConst0 = 0xFFFFFFFEu, kFlatConst1 = 0xFFFFFFFFu;  // con
 constexpr uint32_t kFlatSmem = 227 * 1024;
 constexpr uint32_t kFlatHeader = 512;  // detection state, the queue's item and job
 #if defined(__CUDACC__)
-__host__ __device__
+#define RRTL_FLAT_HD __host__ __device__
+#else
+#define RRTL_FLAT_HD
 #endif
-constexpr uint32_t flat_plane_bytes(uint32_t N) {
+RRTL_FLAT_HD constexpr uint32_t flat_plane_bytes(uint32_t N) {
   return (kFlatSmem - kFlatHeader) / N & ~127u;
+}
+
+// The part of a run that is block `block`'s k-th (n = 0: it has no more): n
+// cycles from c0 of one tile. Tiles laid end to end, each as long as the run's
+// cycles, are cut into equal shares, one a block, so a tile is split between
+// two blocks at most: the later block takes its first cycles before anything
+// else, the earlier one its last cycles after everything else, when those are
+// done (a share is no shorter than a tile).
+struct FlatPart {
+  uint32_t tile;
+  bool first, last;  // the first or last cycles of a split tile
+  uint64_t c0, n;
+};
+RRTL_FLAT_HD inline FlatPart flat_part(uint32_t n_tiles, uint64_t cycles, uint32_t block, uint32_t blocks, uint32_t k) {
+  const uint64_t total = n_tiles * cycles, share = (total + blocks - 1) / blocks;
+  const uint64_t lo = block * share, end = lo + share < total ? lo + share : total;
+  FlatPart p{};
+  if (lo >= total) return p;
+  const uint64_t tile = lo / cycles + k, at = tile * cycles;
+  if (at >= end) return p;
+  p.tile = (uint32_t)tile;
+  p.first = lo > at;
+  p.last = end < at + cycles;
+  p.n = (p.last ? end : at + cycles) - (p.first ? lo : at);
+  p.c0 = p.last ? cycles - p.n : 0;
+  return p;
 }
 
 }  // namespace rrtl

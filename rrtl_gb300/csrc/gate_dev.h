@@ -126,6 +126,7 @@ struct GateRunDev {
   const uint32_t* flat_off0;  // [n_tiles + 1] into flat_forces0
   const uint4* flat_forces0;
   uint32_t flat_serial;       // flat kernel: stimulus may only be stored after the record (a stimulated net is recorded)
+  uint32_t* flat_done;        // flat kernel: [n_tiles], first part of a split tile done (nullptr: no tile is split)
   uint32_t* nets;             // [rows][words_pad]
   uint32_t* err;              // device status word
   unsigned long long cycle_base;  // absolute cycle of the launch's first cycle (stimulus, records)

@@ -420,8 +420,8 @@ uint32_t choose_tile_words(rrtl_design* d, uint32_t words) {
 // 24.8k / 36.9k / 53.9k / 97.8k (sets of one vector: four sets 25.3k / 37.1k
 // / 57.3k / 114k, two sets against two vectors 17.8k / 24.8k / 35.6k /
 // 62.5k). So a tile costs about 220 clocks a level and 9 an entry, and each
-// vector one a wavefront and 75 a level; wide tiles pay until the last round
-// of tiles leaves most SMs idle.
+// vector one a wavefront and 75 a level; wide tiles pay until SMs are left
+// without one.
 constexpr FlatShape kFlatShapes[] = {{4, 2, 2}, {4, 3, 1}, {4, 2, 1}, {4, 1, 1}, {2, 1, 1}, {1, 1, 1}};
 // The tile width a flat run reports: several tiles of the widest documented
 // width that divides its own.
@@ -474,7 +474,8 @@ FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w, uint3
   for (const FlatShape& x : kFlatShapes) {
     if (x.V > top || (x.V == 4 && x.N * x.Q > v->max_n)) continue;
     if (tuned_w && flat_reported_words(x.words()) != tuned_w) continue;
-    const double t = std::ceil(std::ceil((double)words / x.words()) / d->ctx->sm_count) * flat_tile_cost(v->fp, top, x);
+    // (tiles past one a SM are split between blocks: no last round)
+    const double t = std::max(1.0, std::ceil((double)words / x.words()) / d->ctx->sm_count) * flat_tile_cost(v->fp, top, x);
     if (t < best) {
       best = t;
       s = x;
@@ -835,7 +836,7 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
 // closing settle, over the fused variant's.
 GateRunDev flat_run_desc(const GatePrepared& g) {
   GateRunDev R = g.R;
-  R.n_tiles = (g.R.words_pad + g.shape.words() - 1) / g.shape.words();
+  R.n_tiles = (g.R.words + g.shape.words() - 1) / g.shape.words();
   return R;
 }
 GateRunDev closing_desc(const GatePrepared& g) {
@@ -850,18 +851,24 @@ GateRunDev closing_desc(const GatePrepared& g) {
 
 // A flat run: the cycles, then the closing settle, which writes every signal
 // back (with stuck-at forces on the fused kernel).
-void gate_flat_launch(rrtl_design* d, const GatePrepared& g, cudaStream_t st) {
-  const GateRunDev R = flat_run_desc(g), C = closing_desc(g);
-  cuda_check(launch_gate_flat(g.shape.V, g.shape.N, g.shape.Q, g.flat->dev, R, std::min(R.n_tiles, d->ctx->sm_count), st),
-             "gate_flat_kernel");
+void gate_flat_launch(rrtl_batch* b, const GatePrepared& g, cudaStream_t st) {
+  rrtl_design* d = b->d;
+  GateRunDev R = flat_run_desc(g), C = closing_desc(g);
+  const uint32_t grid = std::min(R.n_tiles, d->ctx->sm_count);
+  if (R.n_tiles % grid) {
+    b->d_flat_done.reserve((size_t)R.n_tiles * 4);
+    cuda_check(cudaMemsetAsync(b->d_flat_done.p, 0, (size_t)R.n_tiles * 4, st), "memset flat");
+    R.flat_done = b->d_flat_done.as<uint32_t>();
+  }
+  cuda_check(launch_gate_flat(g.shape.V, g.shape.N, g.shape.Q, g.flat->dev, R, grid, st), "gate_flat_kernel");
   if (g.settle) {
     cuda_check(launch_gate_flat_settle(g.settle_shape.V, g.settle_shape.N, g.settle->dev, C,
                                        std::min(C.n_tiles, d->ctx->sm_count), st),
                "gate_flat_settle_kernel");
     return;
   }
-  const uint32_t grid = std::min<uint32_t>(C.n_tiles, d->ctx->sm_count * g.v->fused_ctas);
-  cuda_check(launch_gate_fused(g.v->gdev, C, grid, g.v->fused_smem, st), "gate_fused_kernel");
+  const uint32_t closing = std::min<uint32_t>(C.n_tiles, d->ctx->sm_count * g.v->fused_ctas);
+  cuda_check(launch_gate_fused(g.v->gdev, C, closing, g.v->fused_smem, st), "gate_fused_kernel");
 }
 
 // Copy a prepared run's recorded outputs to the caller's host buffers.
@@ -981,7 +988,7 @@ void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckT
     cuda_check(launch_gate_jit(*J, g.R, st), "rrtl_gate_jit");
     g.W = 0;
   } else if (g.flat && g.fused) {
-    gate_flat_launch(d, g, st);
+    gate_flat_launch(b, g, st);
     g.W = flat_reported_words(g.shape.words());
   } else if (g.fused) {
     uint32_t grid = std::min<uint32_t>(g.R.n_tiles, d->ctx->sm_count * g.v->fused_ctas);

@@ -275,6 +275,7 @@ struct rrtl_batch {
   rrtl::DevBuf d_nets;
   std::vector<rrtl_fault> faults;
   rrtl::FlatForceTable forces_flat;
+  rrtl::DevBuf d_flat_done;  // per tile of a split run (GateRunDev::flat_done)
   rrtl::ForceTable forces_plain, forces_fused[4];  // plain: 8-word tiles; fused: per log2 W
   // word engine state
   uint32_t lanes_pad = 0;

@@ -34,6 +34,33 @@ uint32_t two(uint32_t meta, uint32_t a, uint32_t b) {
 
 }  // namespace
 
+// Parts of a run over `blocks` blocks: every tile's cycles once and in order, a
+// split tile's first part its block's first, its last part waiting for it and
+// never before the time it is done at equal speed. 0: as stated.
+extern "C" int emu_flat_parts(uint32_t n_tiles, uint64_t cycles, uint32_t blocks) {
+  std::vector<uint64_t> first(n_tiles, 0), last(n_tiles, 0), done(n_tiles, 0);
+  const uint64_t share = (n_tiles * cycles + blocks - 1) / blocks;
+  for (int pass = 0; pass < 2; ++pass)
+    for (uint32_t b = 0; b < blocks; ++b) {
+      uint64_t t = 0;
+      for (uint32_t k = 0;; ++k) {
+        const FlatPart p = flat_part(n_tiles, cycles, b, blocks, k);
+        if (!p.n) break;
+        if (p.tile >= n_tiles || p.c0 + p.n > cycles || (p.first && p.last)) return 1;
+        if (p.first != (p.c0 == 0 && p.n < cycles) || p.last != (p.c0 > 0)) return 2;
+        if (p.first && k) return 3;
+        if (pass == 0) (p.last ? last : first)[p.tile] += p.n;
+        if (p.first) done[p.tile] = p.n;
+        if (pass && p.last && (p.c0 != first[p.tile] || done[p.tile] > t)) return 4;
+        t += p.n;
+      }
+      if (t > share) return 5;
+    }
+  for (uint32_t i = 0; i < n_tiles; ++i)
+    if (first[i] + last[i] != cycles) return 6;
+  return 0;
+}
+
 extern "C" int emu_flat_run(const char* json, size_t len, const char* top, uint32_t V, uint32_t pack, uint32_t fold,
                             uint32_t max_warps, uint32_t max_slots, uint32_t lanes, uint64_t cycles, uint64_t seed,
                             uint64_t lane_base, uint32_t n_stim, const uint32_t* stim_sig, const uint32_t* stim_kind,

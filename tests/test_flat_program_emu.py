@@ -82,6 +82,16 @@ def test_netlist_equals_the_oracle(emu, netlist, V, warps, pack, fold):
     assert st["floor"] <= st["wavefronts"] <= 1.10 * st["floor"], st
 
 
+@pytest.mark.parametrize("blocks", [1, 2, 7, 152])
+def test_split_tiles_cover_a_run_once(emu, blocks):
+    """Tiles past one a block (fewer: one launch of whole tiles), the shortest runs and the longest."""
+    emu.emu_flat_parts.argtypes = [U32, U64, U32]
+    for tiles in [blocks, blocks + 1, blocks + 3, 2 * blocks - 1, 2 * blocks, 3 * blocks + 1, 2048]:
+        for cycles in [4, 5, 7, 100, 2**32 - 1]:
+            if tiles >= blocks:
+                assert emu.emu_flat_parts(tiles, cycles, blocks) == 0, (tiles, cycles)
+
+
 @pytest.mark.parametrize("V", [4, 2, 1])
 def test_closing_settle_writes_every_signal_back(emu, netlist, V):
     """The settle's program alone, its write-backs and the source rows standing for every net."""

@@ -187,3 +187,25 @@ def test_closing_settle_writes_every_signal(wide, monkeypatch, lanes):
         step = 1 if lanes < 5000 else 41
         got.append([g.get_signal_bits(n) for n in (meta.inputs + meta.regs + meta.gate_names)[::step]])
     assert all(np.array_equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("shape,words", [("111", 153), ("111", 301), ("211", 500), ("422", 16 * 171)])
+@pytest.mark.parametrize("cycles", [4, 11])
+def test_tiles_split_between_blocks(wide, monkeypatch, shape, words, cycles):
+    """More tiles than SMs and no multiple: blocks share tiles, every record form, faults detected in either part."""
+    cd, meta, od = wide
+    monkeypatch.setenv("RRTL_FLAT", shape)
+    stim, rec = netlist_run_spec(meta)
+    lanes = 32 * words - 9
+    g = sim.GpuBatchSimulator(cd, lanes=lanes)
+    res = g.run(cycles, seed=6, stim=stim, record=rec[:40], mode=sim.REC_TRACE | sim.REC_HASH)
+    ref = _ref(od, lanes, cycles, 6, stim, rec[:40], 3)
+    assert np.array_equal(res["hash"], ref["hash"]) and np.array_equal(res["trace"], ref["trace"])
+    uni = [(n, sim.STIM_RANDOM_UNIFORM if k == sim.STIM_RANDOM else k, p) for n, k, p in stim]
+    got = []
+    for flat in (shape, "0"):
+        monkeypatch.setenv("RRTL_FLAT", flat)
+        f = sim.GpuBatchSimulator(cd, lanes=lanes)
+        f.set_faults([(ln, meta.gate_names[ln % len(meta.gate_names)], ln & 1) for ln in range(1, lanes, 7) if ln % 32])
+        got.append(f.run(cycles, seed=6, stim=uni, record=rec, mode=sim.REC_DETECT)["detect"])
+    assert np.array_equal(*got) and (got[0] != 0xFFFFFFFF).any()
