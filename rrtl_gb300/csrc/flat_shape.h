@@ -15,6 +15,12 @@ constexpr uint32_t kFlatThreads = kFlatComputeThreads + kFlatServiceThreads;
 constexpr uint32_t kFlatPrefetch = RRTL_FLAT_PREFETCH;  // entries a warp loads ahead
 constexpr uint32_t kFlatMaxVectors = 4;  // vectors per tile of 4-word rows (one for narrower rows)
 constexpr uint64_t kFlatMinCycles = 4;   // shorter runs stay on one launch of the fused kernel
+// One-word rows whose byte offset fits 16 bits are named by it in the entries:
+// a tile-cycle of narrow rows is bound by ALU instructions (two scheduler
+// slots each), of which the address of a row is one less. With the entry
+// batches no longer copied (flat_tile), a tile-cycle of one word takes 25.9k
+// -> 24.6k clocks at 50,000 gates, 70.5k -> 66.9k at 200,000.
+constexpr uint32_t kFlatByteRows = 1u << 14;
 // Entry flags (bits of word y): a level barrier before it, three-input cells.
 constexpr uint32_t kFlatDevSync = 1u << 16, kFlatDevThree = 1u << 24;
 constexpr uint32_t kFlatConst0 = 0xFFFFFFFEu, kFlatConst1 = 0xFFFFFFFFu;  // constant rows of the commit list

@@ -99,6 +99,7 @@ struct FlatProgDev {
   const uint32_t* src_slot;
   const GateRegDev* commit;    // rows (kFlatConst0/1: a constant)
   uint32_t n_src, n_commit, n_slots, warps;
+  uint32_t row_bytes;          // 1: the entries' rows are byte offsets (one-word rows, under 64 KB of them)
 };
 
 struct GateRunDev {

@@ -155,10 +155,10 @@ __device__ __forceinline__ void flat_bar_service() {
   asm volatile("bar.sync 1, %0;" ::"n"(kFlatServiceThreads) : "memory");
 }
 
-// Rows of a cell: byte offsets from the slot array.
-template <int V>
+// Row `slot` of the slot array (kBytes: its byte offset).
+template <int V, bool kBytes>
 __device__ __forceinline__ const typename FlatVec<V>::T* flat_row(const uint8_t* S, uint32_t slot) {
-  return reinterpret_cast<const typename FlatVec<V>::T*>(S + slot * (V * 4u));
+  return reinterpret_cast<const typename FlatVec<V>::T*>(S + (kBytes ? slot : slot * (V * 4u)));
 }
 
 // Entries of two cells per lane (two inputs) and one cell per lane (three
@@ -167,18 +167,18 @@ __device__ __forceinline__ const typename FlatVec<V>::T* flat_row(const uint8_t*
 // compiler cannot know). Functions and row addresses are decoded before the
 // level barrier the entry may wait for.
 // `out` sees every row vector written: out(which cell, plane, value).
-template <int V, int N, int Q, class Bar, class Out>
+template <int V, int N, int Q, bool kBytes, class Bar, class Out>
 __device__ __forceinline__ void flat_pair2(uint8_t* S, const uint4& r, uint32_t go, const Bar& bar, const Out& out) {
   using T = typename FlatVec<V>::T;
   constexpr uint32_t kStep = flat_plane_bytes(N * Q) / sizeof(T);
   constexpr int H = N > 2 ? 2 : N;  // planes whose operands are in registers at once
   const FlatTwo f(r.y), g(r.w);
-  const T* const pa = flat_row<V>(S, r.x & 0xFFFFu);
-  const T* const pb = flat_row<V>(S, r.x >> 16);
-  const T* const pc = flat_row<V>(S, r.z & 0xFFFFu);
-  const T* const pd = flat_row<V>(S, r.z >> 16);
-  T* const po = const_cast<T*>(flat_row<V>(S, r.y & 0xFFFFu));
-  T* const pq = const_cast<T*>(flat_row<V>(S, r.w & 0xFFFFu));
+  const T* const pa = flat_row<V, kBytes>(S, r.x & 0xFFFFu);
+  const T* const pb = flat_row<V, kBytes>(S, r.x >> 16);
+  const T* const pc = flat_row<V, kBytes>(S, r.z & 0xFFFFu);
+  const T* const pd = flat_row<V, kBytes>(S, r.z >> 16);
+  T* const po = const_cast<T*>(flat_row<V, kBytes>(S, r.y & 0xFFFFu));
+  T* const pq = const_cast<T*>(flat_row<V, kBytes>(S, r.w & 0xFFFFu));
   bar.pass(go);
 #pragma unroll
   for (int p0 = 0; p0 < N; p0 += H) {
@@ -203,16 +203,16 @@ __device__ __forceinline__ void flat_pair2(uint8_t* S, const uint4& r, uint32_t 
   }
 }
 
-template <int V, int N, int Q, class Bar, class Out>
+template <int V, int N, int Q, bool kBytes, class Bar, class Out>
 __device__ __forceinline__ void flat_one3(uint8_t* S, const uint4& r, uint32_t go, const Bar& bar, const Out& out) {
   using T = typename FlatVec<V>::T;
   constexpr uint32_t kStep = flat_plane_bytes(N * Q) / sizeof(T);
   constexpr int H = N > 2 ? 2 : N;
   const FlatThree f(r.w);
-  const T* const pa = flat_row<V>(S, r.x & 0xFFFFu);
-  const T* const pb = flat_row<V>(S, r.x >> 16);
-  const T* const pc = flat_row<V>(S, r.z);
-  T* const po = const_cast<T*>(flat_row<V>(S, r.y & 0xFFFFu));
+  const T* const pa = flat_row<V, kBytes>(S, r.x & 0xFFFFu);
+  const T* const pb = flat_row<V, kBytes>(S, r.x >> 16);
+  const T* const pc = flat_row<V, kBytes>(S, r.z);
+  T* const po = const_cast<T*>(flat_row<V, kBytes>(S, r.y & 0xFFFFu));
   bar.pass(go);
 #pragma unroll
   for (int p0 = 0; p0 < N; p0 += H) {
@@ -343,8 +343,8 @@ __device__ __forceinline__ void flat_settle_tile(const FlatProgDev& P, const Gat
           if (net != 0xFFFFFFFFu && col < R.words_pad) *reinterpret_cast<T*>(R.nets + (size_t)net * R.words_pad + col) = v;
         };
         const uint32_t go = r.y & kFlatDevSync;
-        if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, 1>(S, r, go, bar, out);
-        else flat_pair2<V, N, 1>(S, r, go, bar, out);
+        if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, 1, false>(S, r, go, bar, out);
+        else flat_pair2<V, N, 1, false>(S, r, go, bar, out);
       }
 #pragma unroll
       for (int d = 0; d < D; ++d) {
@@ -361,7 +361,7 @@ __device__ __forceinline__ void flat_settle_tile(const FlatProgDev& P, const Gat
 // stuck-at forces; kFull: the program has a stream for every warp of a set.
 // Source nets are read from and written back to the run's global rows; the
 // caller settles the other nets (the closing settle) afterwards.
-template <int V, int N, int Q, bool F, bool kFull>
+template <int V, int N, int Q, bool F, bool kFull, bool kBytes>
 __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev& R, uint32_t tile, uint64_t c0,
                                           uint64_t ncyc, uint8_t* smem) {
   constexpr uint32_t W = V * N * Q;
@@ -414,27 +414,44 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
     for (uint64_t c = 0; c < ncyc; ++c) {
       uint32_t level = 0;
       if constexpr (F) forces.begin(lane, false);
-      for (uint32_t e = 0; e < n; e += D) {
+      // entries [e, e + D) from `cur`, the D after them (the next cycle's first behind the last) into `nx`
+      auto batch = [&](const uint4 (&cur)[D], uint4 (&nx)[D], uint32_t e) {
         const uint4* const ahead = base + (size_t)(e + D < n ? e + D : 0u) * 32u;
-        uint4 nx[D];
 #pragma unroll
         for (int d = 0; d < D; ++d) nx[d] = flat_load_entry(ahead + d * 32);
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-          const uint4 r = q[d];
+          const uint4 r = cur[d];
           const uint32_t go = r.y & kFlatDevSync;
           if constexpr (F) {
             if (go) forces.apply(S, level, lane);  // the same on every lane
           }
           // (the vote makes the branch a warp-uniform one)
-          if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, Q>(Sq, r, go, bar, FlatNoOut{});
-          else flat_pair2<V, N, Q>(Sq, r, go, bar, FlatNoOut{});
+          if (__any_sync(0xFFFFFFFFu, r.y & kFlatDevThree)) flat_one3<V, N, Q, kBytes>(Sq, r, go, bar, FlatNoOut{});
+          else flat_pair2<V, N, Q, kBytes>(Sq, r, go, bar, FlatNoOut{});
           if constexpr (F) {
             if (go) forces.advance(level++);
           }
         }
+      };
+      uint4 nx[D];
+      if constexpr (V < 4 && !F) {
+        // narrow rows are bound by the instructions of an entry: two batches a turn, in place of the copies
+        for (uint32_t e = 0; e < n; e += 2 * D) {
+          batch(q, nx, e);
+          if (e + D < n) {
+            batch(nx, q, e + D);
+          } else {
 #pragma unroll
-        for (int d = 0; d < D; ++d) q[d] = nx[d];
+            for (int d = 0; d < D; ++d) q[d] = nx[d];
+          }
+        }
+      } else {
+        for (uint32_t e = 0; e < n; e += D) {
+          batch(q, nx, e);
+#pragma unroll
+          for (int d = 0; d < D; ++d) q[d] = nx[d];
+        }
       }
       for (uint32_t k = tail; k; --k) {
         if constexpr (F) forces.apply(S, level, lane);

@@ -326,7 +326,22 @@ FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe, 
       const uint32_t fl = (r.has_reset ? 1u : 0u) | (r.active_low ? 2u : 0u) | (r.reset_value ? 4u : 0u);
       commit.push_back(GateRegDev{row(r.q_net), row(r.d_net), r.has_reset ? row(r.rst_net) : kFlatConst0, fl});
     }
-    upload(v->d_stream, fp.stream);
+    // one-word rows whose byte offsets fit an entry's 16 bits are stored as such
+    const bool bytes = V == 1 && !settle && fp.n_slots <= kFlatByteRows;
+    if (bytes) {
+      std::vector<FlatLane> stream(fp.stream);
+      for (FlatLane& l : stream) {
+        const bool three = l.y & kFlatDevThree;
+        l.x <<= 2;  // both rows: their top two bits are clear
+        l.y = (l.y & 0xFFFF0000u) | (l.y & 0x3FFFu) << 2;
+        l.z <<= 2;
+        if (!three) l.w = (l.w & 0xFFFF0000u) | (l.w & 0x3FFFu) << 2;
+      }
+      upload(v->d_stream, stream);
+    } else {
+      upload(v->d_stream, fp.stream);
+    }
+    v->dev.row_bytes = bytes ? 1u : 0u;
     upload(v->d_stream_net, fp.stream_net);
     upload(v->d_warps, warps);
     upload(v->d_src_net, fp.source_nets);

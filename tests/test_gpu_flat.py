@@ -209,3 +209,17 @@ def test_tiles_split_between_blocks(wide, monkeypatch, shape, words, cycles):
         f.set_faults([(ln, meta.gate_names[ln % len(meta.gate_names)], ln & 1) for ln in range(1, lanes, 7) if ln % 32])
         got.append(f.run(cycles, seed=6, stim=uni, record=rec, mode=sim.REC_DETECT)["detect"])
     assert np.array_equal(*got) and (got[0] != 0xFFFFFFFF).any()
+
+
+@pytest.mark.parametrize("shape", ["111", "211"])
+def test_more_rows_than_byte_offsets_name(engine, monkeypatch, shape):
+    """Over 16,384 one-word rows: entries hold row numbers instead of byte offsets."""
+    d, meta = gate_netlist(n_gates=20_000, n_ff=16_500, n_pi=8, n_po=8, depth=6, seed=3)
+    js = d.to_json()
+    od = ob.OracleDesign(js, meta.top)
+    monkeypatch.setenv("RRTL_FLAT", shape)
+    stim, rec = netlist_run_spec(meta)
+    g = sim.GpuBatchSimulator(sim.CompiledDesign(js, meta.top), lanes=70)
+    res = g.run(6, seed=9, stim=stim, record=rec, mode=sim.REC_HASH)
+    assert g.tile_words == int(shape[0])
+    assert np.array_equal(res["hash"], _ref(od, 70, 6, 9, stim, rec, 2)["hash"])
