@@ -9,6 +9,13 @@ namespace rrtl {
 constexpr uint32_t kFlatComputeThreads = 512;  // 16 compute warps (flatprog.h kFlatWarps)
 constexpr uint32_t kFlatServiceThreads = 128;
 constexpr uint32_t kFlatThreads = kFlatComputeThreads + kFlatServiceThreads;
+// Tiles of one or two words (without forces) need so few registers that a run
+// of its own takes 24 compute warps: 50,000 gates 24.6k -> 23.7k (one word)
+// and 28.7k -> 28.0k clocks a tile-cycle, 200,000 gates 66.9k -> 59.1k and
+// 80.9k -> 74.3k; 28 warps are slower again (65.8k and 74.8k before the byte
+// offsets, against 63.2k and 74.4k). Programs of few entries a level use the
+// warps they have entries for.
+constexpr uint32_t kFlatNarrowThreads = 768;
 #ifndef RRTL_FLAT_PREFETCH
 #define RRTL_FLAT_PREFETCH 4
 #endif

@@ -31,8 +31,11 @@ __device__ __forceinline__ bool flat_wait_part(const uint32_t* done, uint64_t cy
 // gates, 5,003 x 200 (157 of 1) 3.11 -> 2.91. At 65,536 lanes x 1,000 it makes
 // 171 tiles of 12 words (42.5 ms) better than 128 of 16 (47.0), which leave 24
 // SMs without a tile.
+template <int V, bool F>
+constexpr uint32_t flat_compute_threads() { return V < 4 && !F ? kFlatNarrowThreads : kFlatComputeThreads; }
+
 template <int V, int N, int Q, bool F, bool kFull, bool kBytes>
-__global__ void __launch_bounds__(kFlatThreads, 1) gate_flat_kernel(FlatProgDev P, GateRunDev R) {
+__global__ void __launch_bounds__(flat_compute_threads<V, F>() + kFlatServiceThreads, 1) gate_flat_kernel(FlatProgDev P, GateRunDev R) {
   extern __shared__ __align__(128) uint8_t smem[];
   for (uint32_t k = 0;; ++k) {
     FlatPart p{};
@@ -47,7 +50,7 @@ __global__ void __launch_bounds__(kFlatThreads, 1) gate_flat_kernel(FlatProgDev 
       if (threadIdx.x == 0) atomicExch(R.err, (uint32_t)RRTL_E_TIMEOUT);
       break;
     }
-    flat_tile<V, N, Q, F, kFull, kBytes>(P, R, p.tile, R.cycle_base + p.c0, p.n, smem);
+    flat_tile<V, N, Q, F, kFull, kBytes, flat_compute_threads<V, F>()>(P, R, p.tile, R.cycle_base + p.c0, p.n, smem);
     if (p.first && threadIdx.x == 0) {
       __threadfence();  // the tile's state, written before flat_tile's last barrier
       asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(R.flat_done + p.tile), "r"(1u) : "memory");
@@ -59,24 +62,25 @@ template <int V, int N, int Q, bool F, bool kFull, bool kBytes>
 static cudaError_t launch_f(const FlatProgDev& P, const GateRunDev& R, uint32_t grid, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(gate_flat_kernel<V, N, Q, F, kFull, kBytes>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlatSmem);
   if (e != cudaSuccess) return e;
+  constexpr uint32_t threads = flat_compute_threads<V, F>() + kFlatServiceThreads;
   if (R.flat_done) {
     // blocks wait for one another: all of them resident, or whole tiles
     void* args[] = {const_cast<FlatProgDev*>(&P), const_cast<GateRunDev*>(&R)};
-    e = cudaLaunchCooperativeKernel(gate_flat_kernel<V, N, Q, F, kFull, kBytes>, dim3(grid), dim3(kFlatThreads), args, kFlatSmem, st);
+    e = cudaLaunchCooperativeKernel(gate_flat_kernel<V, N, Q, F, kFull, kBytes>, dim3(grid), dim3(threads), args, kFlatSmem, st);
     if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported) return e;
     cudaGetLastError();
     GateRunDev whole = R;
     whole.flat_done = nullptr;
-    gate_flat_kernel<V, N, Q, F, kFull, kBytes><<<grid, kFlatThreads, kFlatSmem, st>>>(P, whole);
+    gate_flat_kernel<V, N, Q, F, kFull, kBytes><<<grid, threads, kFlatSmem, st>>>(P, whole);
     return cudaGetLastError();
   }
-  gate_flat_kernel<V, N, Q, F, kFull, kBytes><<<grid, kFlatThreads, kFlatSmem, st>>>(P, R);
+  gate_flat_kernel<V, N, Q, F, kFull, kBytes><<<grid, threads, kFlatSmem, st>>>(P, R);
   return cudaGetLastError();
 }
 
 template <int V, int N, int Q>
 static cudaError_t launch(const FlatProgDev& P, const GateRunDev& R, uint32_t grid, cudaStream_t st) {
-  const bool full = P.warps == kFlatComputeThreads / 32 / Q;
+  const bool full = P.warps == flat_compute_threads<V, false>() / 32 / Q;
   if constexpr (V == 1) {
     if (P.row_bytes) {
       if (R.has_forces) return launch_f<V, N, Q, true, false, true>(P, R, grid, st);
@@ -136,13 +140,13 @@ __device__ __forceinline__ void queue_tile(const FlatJobDev& J, const GateItemDe
   }
   if constexpr (V == 1) {
     if (J.P.row_bytes) {
-      if (J.R.has_forces) flat_tile<V, N, Q, true, false, true>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
-      else flat_tile<V, N, Q, false, false, true>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
+      if (J.R.has_forces) flat_tile<V, N, Q, true, false, true, kFlatComputeThreads>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
+      else flat_tile<V, N, Q, false, false, true, kFlatComputeThreads>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
       return;
     }
   }
-  if (J.R.has_forces) flat_tile<V, N, Q, true, false, false>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
-  else flat_tile<V, N, Q, false, false, false>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
+  if (J.R.has_forces) flat_tile<V, N, Q, true, false, false, kFlatComputeThreads>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
+  else flat_tile<V, N, Q, false, false, false, kFlatComputeThreads>(J.P, J.R, item.tile, item.c0, item.ncyc, smem);
 }
 
 __global__ void __launch_bounds__(kFlatThreads, 1) gate_flat_queue_kernel(FlatQueueDev L) {

@@ -18,10 +18,11 @@
 // behind, the integer pipe (3 LOP3 a two-input cell word, 7 a three-input
 // one). 50,000 gates, one tile per SM, clocks per 32-lane word and cycle: 6.0k
 // at 16 words (4.1k of them wavefronts), 6.4k at 12, 6.9k at 8, 9.2k at 4,
-// 14.5k at 2, 25.7k at 1; the fused kernel compiled for the design took 10.1k at 8.
-// 65,536 lanes x 1,000 cycles: 79.5 -> 47.9 ms with the closing settle and
-// the flip-flop read-back; 200 lanes x 100 cycles 2.97 -> 1.56 ms; 200,000
-// gates, 10,007 lanes x 100 cycles 20.4 -> 7.85 ms (rows of 4 words fit now).
+// 14.0k at 2, 23.7k at 1; the fused kernel compiled for the design took 10.1k at 8.
+// 65,536 lanes x 1,000 cycles: 79.6 -> 42.5 ms with the closing settle and
+// the flip-flop read-back (47.9 before tiles were split between blocks); 200
+// lanes x 100 cycles 2.97 -> 1.29 ms; 200,000 gates, 10,007 lanes x 100 cycles
+// 20.4 -> 5.0 ms.
 //
 // What decided the form, 50,000 gates at 8 words, clocks per tile-cycle: entry
 // loads issued one by one into a rotating queue 85.6k (each waits behind the
@@ -281,9 +282,10 @@ struct FlatForces {
   __device__ __forceinline__ uint32_t last() const { return __shfl_sync(0xFFFFFFFFu, f.w, 31); }
 };
 
+template <int kCompute>
 __device__ __forceinline__ void flat_bar_compute() {
   __syncwarp();
-  asm volatile("bar.sync 6, %0;" ::"n"(kFlatComputeThreads) : "memory");
+  asm volatile("bar.sync 6, %0;" ::"n"(kCompute) : "memory");
 }
 
 // Source rows of a tile of W words in (words past the padded batch read as zero).
@@ -358,10 +360,11 @@ __device__ __forceinline__ void flat_settle_tile(const FlatProgDev& P, const Gat
 }
 
 // Cycles [c0, c0 + ncyc) of one tile (V * N * Q words) of a run; F: with
-// stuck-at forces; kFull: the program has a stream for every warp of a set.
+// stuck-at forces; kFull: the program has a stream for every warp of a set;
+// kBytes: its entries hold byte offsets; kCompute: compute threads.
 // Source nets are read from and written back to the run's global rows; the
 // caller settles the other nets (the closing settle) afterwards.
-template <int V, int N, int Q, bool F, bool kFull, bool kBytes>
+template <int V, int N, int Q, bool F, bool kFull, bool kBytes, int kCompute>
 __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev& R, uint32_t tile, uint64_t c0,
                                           uint64_t ncyc, uint8_t* smem) {
   constexpr uint32_t W = V * N * Q;
@@ -386,11 +389,11 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
   }
   __syncthreads();
   const bool serial = F || P.n_commit != 0 || R.flat_serial;
-  if (tid < kFlatComputeThreads) {
-    constexpr uint32_t kSetWarps = kFlatComputeThreads / 32 / Q;
-    const uint32_t set = Q == 1 ? 0u : tid / (kFlatComputeThreads / Q), warp = (tid >> 5) % kSetWarps;
+  if (tid < kCompute) {
+    constexpr uint32_t kSetWarps = kCompute / 32 / Q;
+    const uint32_t set = Q == 1 ? 0u : tid / (kCompute / Q), warp = (tid >> 5) % kSetWarps;
     uint8_t* const Sq = S + set * (N * kPlane);  // the set's planes
-    const FlatBar<kFull ? (int)(kFlatComputeThreads / Q) : 0> bar{2u + set, P.warps * 32u};
+    const FlatBar<kFull ? kCompute / Q : 0> bar{2u + set, P.warps * 32u};
     const bool active = warp < P.warps;  // a program of few cells a level has fewer streams than the set has warps
     const uint32_t begin = active ? __ldg(P.warp_begin + warp) : 0u, n = active ? __ldg(P.warp_begin + warp + 1) - begin : 0u;
     const uint32_t tail = active ? __ldg(P.warp_tail + warp) : 0u;
@@ -462,7 +465,7 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
       __syncthreads();  // every level done
       if (serial) {
         // registers left on the commit list
-        for (uint32_t i = tid; i < P.n_commit * W; i += kFlatComputeThreads) {
+        for (uint32_t i = tid; i < P.n_commit * W; i += kCompute) {
           const uint4 rr = __ldg(reinterpret_cast<const uint4*>(P.commit) + i / W);
           const uint32_t ww = i % W;
           uint32_t d = rr.y == kFlatConst0 ? 0u : rr.y == kFlatConst1 ? 0xFFFFFFFFu : word_at(rr.y, ww);
@@ -474,8 +477,8 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
           word_at(rr.x, ww) = d;
         }
         if constexpr (F) {
-          if (P.n_commit) flat_bar_compute();
-          for (uint32_t i = begin0 + tid; i < end0; i += kFlatComputeThreads) {
+          if (P.n_commit) flat_bar_compute<kCompute>();
+          for (uint32_t i = begin0 + tid; i < end0; i += kCompute) {
             const uint4 f = i == begin0 + tid ? first0 : __ldg(R.flat_forces0 + i);
             uint32_t& v = *reinterpret_cast<uint32_t*>(S + f.x);
             v = (v & ~f.y) | (f.z & f.y);
@@ -486,7 +489,7 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
       __syncthreads();  // next cycle's stimulus in place
     }
   } else {
-    const uint32_t st = tid - kFlatComputeThreads;
+    const uint32_t st = tid - kCompute;
     constexpr int KS = 10, KR = 8;  // stimulus and record words a thread holds in registers
     const uint32_t n_stim = R.n_stim * W, n_rec = R.n_rec * W;
     uint32_t sv[KS], rv[KR];

@@ -279,12 +279,10 @@ GateVariant* gate_variant(rrtl_design* d, uint32_t W) {
   return d->gvar[li].get();
 }
 
-// Build and upload the flat program of row width V for Q warp sets; observe:
-// with a row for every signal (runs with stuck-at forces); settle: the closing settle's.
-FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe, bool settle = false) {
+// Build and upload the flat program of row width V for Q warp sets.
+FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, FlatKind kind) {
   std::lock_guard<std::mutex> lk(d->gvar_mu);
-  std::unique_ptr<FlatVariant>& slot =
-      settle ? d->fvar_settle[log2_words(V)] : d->fvar[log2_words(V)][log2_words(Q)][observe ? 1 : 0];
+  std::unique_ptr<FlatVariant>& slot = d->fvar[log2_words(V)][log2_words(Q)][kind];
   if (slot) return slot.get();
   auto v = std::make_unique<FlatVariant>();
   const GateProgram& gp = d->gp();
@@ -296,9 +294,9 @@ FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe, 
     return slots <= kMaxSlots && d->ctx->max_smem >= kFlatSmem ? n : 0u;
   };
   FlatOptions o;
-  o.max_warps = kFlatComputeThreads / 32 / Q;
-  o.observe = observe;
-  o.settle = settle;
+  o.max_warps = (kind == kFlatNarrow ? kFlatNarrowThreads : kFlatComputeThreads) / 32 / Q;
+  o.observe = kind == kFlatObserve;
+  o.settle = kind == kFlatSettle;
   v->fp = build_flat_program(gp, V, o);
   v->max_n = fit(v->fp.n_slots);
   if (v->max_n < top) {
@@ -327,7 +325,7 @@ FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, bool observe, 
       commit.push_back(GateRegDev{row(r.q_net), row(r.d_net), r.has_reset ? row(r.rst_net) : kFlatConst0, fl});
     }
     // one-word rows whose byte offsets fit an entry's 16 bits are stored as such
-    const bool bytes = V == 1 && !settle && fp.n_slots <= kFlatByteRows;
+    const bool bytes = V == 1 && kind != kFlatSettle && fp.n_slots <= kFlatByteRows;
     if (bytes) {
       std::vector<FlatLane> stream(fp.stream);
       for (FlatLane& l : stream) {
@@ -429,14 +427,17 @@ uint32_t choose_tile_words(rrtl_design* d, uint32_t words) {
 // forces a shape (A/B switches).
 //
 // The cost of a tile-cycle in SM clocks was fitted to one wave of tiles on
-// netlists of 41 levels and 3,000 / 10,000 / 20,000 / 50,000 gates: one-word
-// rows 10.9k / 12.4k / 15.5k / 26.1k; one 4-word vector 12.9k / 17.4k / 22.7k
+// netlists of 41 levels and 10,000 / 50,000 / 200,000 gates for narrow tiles:
+// one word 12.1k / 24.6k / 66.9k (24 warps 12.1k / 23.7k / 59.1k), two 13.8k /
+// 28.7k / 80.9k (13.8k / 28.0k / 74.3k); and on 3,000 / 10,000 / 20,000 /
+// 50,000 gates: one 4-word vector 12.9k / 17.4k / 22.7k
 // / 37.2k, two 16.4k / 24.8k / 33.5k / 56.1k, four as two warp sets of two
 // 24.8k / 36.9k / 53.9k / 97.8k (sets of one vector: four sets 25.3k / 37.1k
 // / 57.3k / 114k, two sets against two vectors 17.8k / 24.8k / 35.6k /
 // 62.5k). So a tile costs about 220 clocks a level and 9 an entry, and each
 // vector one a wavefront and 75 a level; wide tiles pay until SMs are left
-// without one.
+// without one. (A one-word tile in the queue is priced above its 20.3 clocks an
+// entry: at that price a stream of 24 jobs took 11.5 instead of 11.0 ms.)
 constexpr FlatShape kFlatShapes[] = {{4, 2, 2}, {4, 3, 1}, {4, 2, 1}, {4, 1, 1}, {2, 1, 1}, {1, 1, 1}};
 // The tile width a flat run reports: several tiles of the widest documented
 // width that divides its own.
@@ -446,7 +447,7 @@ uint32_t flat_reported_words(uint32_t w) { return w == 16 ? 8 : w == 12 ? 4 : w;
 // width `base`.
 double flat_tile_cost(const FlatProgram& fp, uint32_t base, const FlatShape& x) {
   const double L = fp.n_levels, E = fp.n_entries;
-  if (x.V != 4) return 173.0 * L + (x.V == 2 ? 25.0 : 21.7) * E;
+  if (x.V != 4) return 173.0 * L + (x.V == 2 ? (x.narrow ? 23.0 : 25.0) : x.narrow ? 18.5 : 21.7) * E;
   const double vec4 = (double)fp.wavefronts * (base == 4 ? 1.0 : base == 2 ? 1.9 : 3.6);  // wavefronts of 4-word rows
   return 222.0 * L + 9.1 * E + x.N * x.Q * (1.03 * vec4 + 75.0 * L);
 }
@@ -455,17 +456,18 @@ double flat_tile_cost(const FlatProgram& fp, uint32_t base, const FlatShape& x) 
 // fused program's slots.
 uint32_t flat_base(rrtl_design* d, bool observe) {
   for (uint32_t V = 4; V >= 1; V /= 2)
-    if ((size_t)d->gp().n_slots * V * 4 <= flat_plane_bytes(1) / 4 * 5 && flat_variant(d, V, 1, observe)->max_n) return V;
+    if ((size_t)d->gp().n_slots * V * 4 <= flat_plane_bytes(1) / 4 * 5 && flat_variant(d, V, 1, observe ? kFlatObserve : kFlatPlain)->max_n) return V;
   return 0;
 }
 
 bool flat_fits(rrtl_design* d, const FlatShape& x, bool observe) {
-  return flat_variant(d, x.V, x.Q, observe)->max_n >= x.N * x.Q;
+  return flat_variant(d, x.V, x.Q, x.narrow ? kFlatNarrow : observe ? kFlatObserve : kFlatPlain)->max_n >= x.N * x.Q;
 }
 
 FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w, uint32_t tuned_w, bool observe) {
   FlatShape s;
   auto checked = [&](FlatShape x) {
+    x.narrow = x.V < 4 && !observe;
     if (x.V && !flat_fits(d, x, observe)) x.V = 0;
     return x;
   };
@@ -484,9 +486,10 @@ FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w, uint3
   }
   const uint32_t top = flat_base(d, observe);
   if (!top) return s;
-  const FlatVariant* v = flat_variant(d, top, 1, observe);
+  const FlatVariant* v = flat_variant(d, top, 1, observe ? kFlatObserve : kFlatPlain);
   double best = INFINITY;
-  for (const FlatShape& x : kFlatShapes) {
+  for (FlatShape x : kFlatShapes) {
+    x.narrow = x.V < 4 && !observe;
     if (x.V > top || (x.V == 4 && x.N * x.Q > v->max_n)) continue;
     if (tuned_w && flat_reported_words(x.words()) != tuned_w) continue;
     // (tiles past one a SM are split between blocks: no last round)
@@ -506,9 +509,9 @@ FlatShape choose_settle(rrtl_design* d, uint32_t words) {
   FlatShape s;
   uint32_t top = 0;
   for (uint32_t V = 4; V >= 1 && !top; V /= 2)
-    if ((size_t)d->gp().n_slots * V * 4 <= flat_plane_bytes(1) / 4 * 5 && flat_variant(d, V, 1, false, true)->max_n) top = V;
+    if ((size_t)d->gp().n_slots * V * 4 <= flat_plane_bytes(1) / 4 * 5 && flat_variant(d, V, 1, kFlatSettle)->max_n) top = V;
   if (!top) return s;
-  const FlatVariant* v = flat_variant(d, top, 1, false, true);
+  const FlatVariant* v = flat_variant(d, top, 1, kFlatSettle);
   double best = INFINITY;
   for (const FlatShape& x : {FlatShape{4, 2, 1}, FlatShape{4, 1, 1}, FlatShape{2, 1, 1}, FlatShape{1, 1, 1}}) {
     if (x.V > top || (x.V == 4 && x.N > v->max_n)) continue;
@@ -518,7 +521,7 @@ FlatShape choose_settle(rrtl_design* d, uint32_t words) {
       s = x;
     }
   }
-  if (s.V && flat_variant(d, s.V, 1, false, true)->max_n < s.N) s.V = 0;
+  if (s.V && flat_variant(d, s.V, 1, kFlatSettle)->max_n < s.N) s.V = 0;
   return s;
 }
 
@@ -686,7 +689,7 @@ bool flat_takes(rrtl_batch* b, const rrtl_run& run) {
   const uint32_t base = flat_base(d, observe);
   if (!base) return false;
   const GateProgram& p = d->gp();
-  const FlatProgram& fp = flat_variant(d, base, 1, observe)->fp;
+  const FlatProgram& fp = flat_variant(d, base, 1, observe ? kFlatObserve : kFlatPlain)->fp;
   for (uint32_t i = 0; i < run.n_record; ++i)
     if (run.record[i] >= p.signal_net.size() || !fp.recordable[p.signal_net[run.record[i]]]) return false;
   for (uint32_t i = 0; observe && i < run.n_stim; ++i)
@@ -715,12 +718,12 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   cudaStream_t st = d->ctx->stream;
   GatePrepared g;
   if (flat.V) {
-    g.flat = flat_variant(d, flat.V, flat.Q, !b->faults.empty());
+    g.flat = flat_variant(d, flat.V, flat.Q, flat.narrow ? kFlatNarrow : b->faults.empty() ? kFlatPlain : kFlatObserve);
     g.shape = flat;
     // the fused kernel's settle applies stuck-at forces; without them the flat
     // one is faster at every size tried (200 to 65,536 lanes, 50k and 200k gates)
     if (b->faults.empty()) g.settle_shape = choose_settle(d, b->words);
-    if (g.settle_shape.V) g.settle = flat_variant(d, g.settle_shape.V, 1, false, true);
+    if (g.settle_shape.V) g.settle = flat_variant(d, g.settle_shape.V, 1, kFlatSettle);
   }
   // (the fused kernel only closes a flat run: the variant built at load time does)
   const uint32_t W = !want_fused ? 0
@@ -1361,7 +1364,7 @@ std::vector<FlatShape> queue_shapes(rrtl_ctx* c, const std::vector<QueueJob*>& j
     if (!flat_takes(b, jobs[i]->run)) continue;
     const bool observe = !b->faults.empty();
     const uint32_t base = flat_base(b->d, observe), tw = tuned_words(b->d, b->words);
-    const FlatVariant* v = flat_variant(b->d, base, 1, observe);
+    const FlatVariant* v = flat_variant(b->d, base, 1, observe ? kFlatObserve : kFlatPlain);
     auto add = [&](FlatShape x) {
       const double len = (double)jobs[i]->run.cycles * flat_tile_cost(v->fp, base, x);
       opts[i].push_back(Choice{x, len, len * std::ceil((double)b->words / x.words())});

@@ -68,6 +68,14 @@ struct GateVariant {
   DevBuf d_srecs, d_pieces, d_src_net, d_src_slot, d_sregs, d_wb, d_grecs, d_lgb, d_gregs;
 };
 
+// What a flat program is for.
+enum FlatKind {
+  kFlatPlain,
+  kFlatObserve,  // a row for every signal: runs with stuck-at forces
+  kFlatNarrow,   // streams for kFlatNarrowThreads: runs on tiles of one or two words, outside the queue
+  kFlatSettle,   // the closing settle
+};
+
 // The flat program for one row width V, with its device copy.
 struct FlatVariant {
   FlatProgram fp;
@@ -80,6 +88,7 @@ struct FlatVariant {
 // warp sets Q.
 struct FlatShape {
   uint32_t V = 0, N = 1, Q = 1;
+  bool narrow = false;  // on the kFlatNarrow program
   uint32_t words() const { return V * N * Q; }
 };
 
@@ -240,8 +249,7 @@ struct rrtl_design {
   // gate engine: one program per fused tile width W (index log2 W), built on
   // demand; nets, levels and registers are the same in every variant
   std::unique_ptr<rrtl::GateVariant> gvar[4];
-  std::unique_ptr<rrtl::FlatVariant> fvar[3][3][2];  // flat programs by log2 V, log2 of the warp sets, with a row for every signal
-  std::unique_ptr<rrtl::FlatVariant> fvar_settle[3];  // closing settles by log2 V
+  std::unique_ptr<rrtl::FlatVariant> fvar[3][3][4];  // flat programs by log2 V, log2 of the warp sets, FlatKind
   uint32_t gate_base = 3;   // log2 W of the variant built at load time
   uint32_t gate_w_max = 0;  // widest W whose slots fit on chip, 0 if none
   std::map<uint32_t, uint32_t> tuned_w;  // measured best W by lane bucket (ceil log2 of 32-lane words);

@@ -70,7 +70,7 @@ def netlist():
     return js, meta, ob.OracleDesign(js, meta.top)
 
 
-@pytest.mark.parametrize("V,warps", [(4, 16), (4, 8), (2, 16), (1, 16)])
+@pytest.mark.parametrize("V,warps", [(4, 16), (4, 8), (2, 16), (1, 16), (2, 24), (1, 24)])
 @pytest.mark.parametrize("pack,fold", [(0, 0), (1, 0), (0, 1), (1, 1), (2, 1)])
 def test_netlist_equals_the_oracle(emu, netlist, V, warps, pack, fold):
     js, meta, od = netlist
