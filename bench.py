@@ -1102,10 +1102,10 @@ def main():
     # is 128 bytes per clock per SM
     sm_mhz = clock_summary.get("sm_mhz") or 2070.0
     smem_peak = ctx.sm_count * 128.0 * sm_mhz * 1e6 / 1e9
-    issue = profiled_issue("gate_fused_kernel_c2.md")
+    issue = profiled_issue("gate_flat_kernel_c2.md")
     # DRAM traffic of one launch grows with lanes (closing write-back of every
     # net), not with cycles (per-cycle work stays in shared memory and L2)
-    traffic, tlanes = profiled_traffic("gate_fused_kernel_c2.md")
+    traffic, tlanes = profiled_traffic("gate_flat_kernel_c2.md")
     if traffic is not None:
         traffic = traffic * LANES / tlanes
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -1130,8 +1130,7 @@ def main():
                                f"window {WINDOW}", "lanes_per_gpu": LANES, "cycles_per_step": CYCLES,
                    "global_lanes": LANES * ws, "parallelism": f"lane shards x{ws} (no collective; rank r simulates "
                                                      f"global lanes [r*{LANES}, (r+1)*{LANES}) of one run)",
-                   "l2": "lane state 428 MB > 129 MB L2 (no flush)", "path": ("fused persistent kernel (generic: RRTL_FUSED_JIT=0)" if os.environ.get("RRTL_FUSED_JIT", "1")[:1] == "0"
-                            else "fused persistent kernel compiled for the design's truth-table classes (NVRTC)"),
+                   "l2": "lane state 428 MB > 129 MB L2 (no flush)", "path": "flat gate kernel (all cycles in one launch), then its closing settle",
                    "tile_words": tile_words},
         "gate_evals_per_s": value * info.n_gates,
         "design": {"gates": info.n_gates, "levels": info.n_levels, "nets": info.n_nets, "slots": info.n_slots,
@@ -1140,7 +1139,7 @@ def main():
         "e2e_host_trace": e2e_trace,
         "plain_path": plain,
         "roofline": roofline,
-        "gpu_launches": args.steps,
+        "gpu_launches": 2 * args.steps,  # the cycles and the closing settle
         "clocks": clock_summary,
         "parity": parity,
     }
