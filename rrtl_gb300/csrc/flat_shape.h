@@ -6,7 +6,7 @@
 
 namespace rrtl {
 
-constexpr uint32_t kFlatComputeThreads = 512;  // 16 compute warps (flatprog.h kFlatWarps)
+constexpr uint32_t kFlatComputeThreads = 512;  // 16 compute warps
 constexpr uint32_t kFlatServiceThreads = 128;
 constexpr uint32_t kFlatThreads = kFlatComputeThreads + kFlatServiceThreads;
 // Tiles of one or two words (without forces) need so few registers that a run

@@ -9,9 +9,9 @@
 //  1. Packing: within a cycle only the recorded and committed nets can be
 //     observed, so inverters and buffers are folded into their readers and a
 //     net with a single reader is folded into that reader where the result
-//     still has at most three inputs. (The closing settle, which writes every
-//     signal back, runs on the fused kernel; for runs with stuck-at forces
-//     FlatOptions::observe keeps a row for every signal.)
+//     still has at most three inputs. (FlatOptions::settle: the closing
+//     settle's program, which computes every signal and writes it back;
+//     FlatOptions::observe: a row for every signal, for stuck-at forces.)
 //  2. Register folding: a cell that computes a register's next value writes
 //     the register's own row, with the synchronous reset in its function, at
 //     a level after every other read of the register. Registers for which

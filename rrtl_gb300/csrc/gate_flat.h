@@ -1,7 +1,8 @@
 // Device code of the flat gate kernel: cycles of a flat gate program
 // (flatprog.h) over tiles of N vectors of V words.
 //
-// One CTA per SM: 16 compute warps walk the levels, four service warps prepare
+// One CTA per SM: 16 compute warps (24 for tiles of one or two words) walk the
+// levels, four service warps prepare
 // the next cycle's stimulus and finish the last cycle's record (hash, trace,
 // detection) while the levels run, so a cycle boundary is two barriers and
 // the row copies. Rows ("slots") are V words; the vectors of a tile lie in

@@ -851,7 +851,7 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
 }
 
 // Descriptors of a flat run's cycles, over the flat shape's tiles, and of its
-// closing settle, over the fused variant's.
+// closing settle, over its own shape's or the fused variant's.
 GateRunDev flat_run_desc(const GatePrepared& g) {
   GateRunDev R = g.R;
   R.n_tiles = (g.R.words + g.shape.words() - 1) / g.shape.words();

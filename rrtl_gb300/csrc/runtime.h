@@ -113,7 +113,7 @@ struct GatePrepared {
   GateRunTables tables;  // host copies of the run's stimulus and record tables
   bool fused = false;
   uint32_t W = 0;
-  // the flat kernel runs the cycles and the fused kernel the closing settle
+  // the flat kernel's program and shape (nullptr: the run is not on it)
   FlatVariant* flat = nullptr;
   FlatShape shape;
   // flat form of the closing settle (nullptr: the fused kernel's)
