@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import json
+import operator
 import os
 from ctypes import POINTER, byref, c_char_p, c_float, c_int32, c_size_t, c_uint32, c_uint64, c_void_p
 from typing import Iterable, Optional, Sequence, Union
@@ -508,18 +509,17 @@ class CompiledDesign:
             self._engine = self.info.engine
         return self._engine
 
+    def index(self, s) -> int:
+        """Packed index of a signal given by name (or index)."""
+        if isinstance(s, str):
+            return (self._cache.get(s) or self.signal(s))[0]
+        if isinstance(s, int):
+            return s
+        raise TypeError("signals are addressed by name or packed index")
+
     def indices(self, signals) -> np.ndarray:
-        """Packed indices of signals given by name (or index)."""
-        cache = self._cache
-        out = []
-        for s in signals:
-            if isinstance(s, str):
-                out.append((cache.get(s) or self.signal(s))[0])
-            elif isinstance(s, int):
-                out.append(s & 0xFFFFFFFF)
-            else:
-                raise TypeError("signals are addressed by name or packed index")
-        return np.array(out, dtype=np.uint32)
+        """Packed indices of signals given by name (or index); OverflowError for an index outside 32 bits."""
+        return np.array([self.index(s) for s in signals], dtype=np.uint32)
 
     def signal(self, name: str):
         """(index, width, kind) of a signal by name."""
@@ -730,13 +730,10 @@ class GpuBatchSimulator:
     def make_run(self, cycles: int, seed: int = 0, stim: Iterable = (), record: Iterable = (), mode: int = 0,
                  input_trace: Optional[np.ndarray] = None, out_trace=None, out_hash=None, detect=None,
                  lane_base: int = 0) -> Run:
-        st = list(stim)
-        arr = np.zeros(max(1, len(st)), dtype=_STIM_DTYPE)
-        if st:
-            names, kinds, params = zip(*st)
-            arr["signal"] = self.design.indices(names)
-            arr["kind"] = np.array([k & 0xFFFFFFFF for k in kinds], dtype=np.uint32)
-            arr["param"] = np.array([p & 0xFFFFFFFFFFFFFFFF for p in params], dtype=np.uint64)
+        # any integer (a NumPy scalar too), reduced to its field's width as a C structure takes it
+        st = [(self.design.index(s) & 0xFFFFFFFF, operator.index(k) & 0xFFFFFFFF, operator.index(p) & 0xFFFFFFFFFFFFFFFF)
+              for s, k, p in stim]
+        arr = np.array(st or [(0, 0, 0)], dtype=_STIM_DTYPE)
         rec = self.design.indices(record)
         r = Run()
         r.cycles = cycles
