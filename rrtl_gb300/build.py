@@ -44,6 +44,7 @@ JIT_HEADERS = [
     ("word_lane.h", "word_lane.h"),
     ("word_dev.h", "word_dev.h"),
     ("stim.h", "stim.h"),
+    ("lanes.h", "lanes.h"),
     ("check_log.h", "check_log.h"),
     ("gate_dev.h", "gate_dev.h"),
     ("gate_common.h", "gate_common.h"),

@@ -9,6 +9,7 @@
 #include "../../include/rrtl_cuda.h"
 #include "check_log.h"
 #include "gate_dev.h"
+#include "lanes.h"
 #include "stim.h"
 
 namespace rrtl {
@@ -19,14 +20,6 @@ __device__ __forceinline__ uint32_t lop3(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
   asm("lop3.b32 %0, %1, %2, %3, %4;" : "=r"(d) : "r"(a), "r"(b), "r"(c), "n"(L));
   return d;
-}
-
-// Lanes of 32-lane word gw that exist in a batch of `lanes` lanes.
-__device__ __forceinline__ uint32_t valid_mask(uint32_t gw, uint32_t lanes) {
-  uint32_t base = gw * 32u;
-  if (base >= lanes) return 0u;
-  uint32_t n = lanes - base;
-  return n >= 32u ? 0xFFFFFFFFu : ((1u << n) - 1u);
 }
 
 __device__ __forceinline__ uint32_t stim_value(const GateStimDev& s, const GateRunDev& R, uint64_t c, uint32_t gw,

@@ -381,12 +381,8 @@ __device__ __forceinline__ void flat_tile(const FlatProgDev& P, const GateRunDev
   flat_load_sources<V, W, kPlane>(P, R, col0, S);
   if (tid < 16u) {
     // lanes already detected by an earlier part of this run stay detected
-    uint32_t det = 0u;
-    if ((R.mode & RRTL_REC_DETECT) && tid < W && col0 + tid < R.words)
-      for (uint32_t b = 0; b < 32u; ++b)
-        if (R.detect[(col0 + tid) * 32u + b] != 0xFFFFFFFFu) det |= 1u << b;
     dstate[tid] = 0u;
-    dstate[16 + tid] = det;
+    dstate[16 + tid] = (R.mode & RRTL_REC_DETECT) && tid < W ? detected_lanes(R.detect, col0 + tid, R.lanes) : 0u;
   }
   __syncthreads();
   const bool serial = F || P.n_commit != 0 || R.flat_serial;

@@ -416,12 +416,8 @@ __device__ __forceinline__ void fused_tile(const GateProgDev& P, const GateRunDe
   }
   if (tid < 8u) {
     // lanes already detected by an earlier part of this run stay detected
-    uint32_t det = 0u;
-    if ((R.mode & RRTL_REC_DETECT) && tid < W && col0 + tid < R.words)
-      for (uint32_t b = 0; b < 32u; ++b)
-        if (R.detect[(col0 + tid) * 32u + b] != 0xFFFFFFFFu) det |= 1u << b;
     dstate[tid] = 0u;
-    dstate[8 + tid] = det;
+    dstate[8 + tid] = (R.mode & RRTL_REC_DETECT) && tid < W ? detected_lanes(R.detect, col0 + tid, R.lanes) : 0u;
   }
   for (uint32_t i = tid; i < P.n_src * W; i += blockDim.x) {
     uint32_t k = i / W, ww = i % W;

@@ -142,9 +142,8 @@ std::string gate_jit_source(const GateProgram& gp, const GateRunTables& run, uin
     o += "      if (t) atomicAdd(R.out_hash + (R.cycle_base + e - lane), t);\n    }\n  };\n";
   }
   auto detect_state = [&](const char* cond) {
-    o += "    uint32_t det = 0u;  // lanes detected by an earlier launch of the run stay detected\n";
-    o += std::string("    if (") + cond + "w < R.words)\n      for (uint32_t b = 0; b < 32u; ++b)\n";
-    o += "        if (R.detect[w * 32u + b] != 0xFFFFFFFFu) det |= 1u << b;\n";
+    // lanes detected by an earlier launch of the run stay detected
+    o += std::string("    uint32_t det = ") + cond + "detected_lanes(R.detect, w, R.lanes)" + (*cond ? " : 0u" : "") + ";\n";
   };
   const std::string detect_end =
       "        uint32_t nb = w < R.words ? diff & ~det & vm : 0u;\n        det |= nb;\n"
@@ -157,7 +156,7 @@ std::string gate_jit_source(const GateProgram& gp, const GateRunTables& run, uin
     o += "  if (warp != 0u) {\n";
     o += "    const uint32_t me = warp - 1u;\n";
     if (nr) o += "    const uint32_t vm = valid_mask(w, R.lanes);\n";
-    if (nr && detect) detect_state("me == 0u && ");
+    if (nr && detect) detect_state("me == 0u ? ");
     if (ns) {
       o += "    if (me == 0u && lane == 0u) {\n";
       for (size_t i = 0; i < ns; ++i) {
