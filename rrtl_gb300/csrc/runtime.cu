@@ -474,10 +474,9 @@ FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w, uint3
   const char* env = getenv("RRTL_FLAT");
   if (env && env[0] == '0') return s;
   if (env && strlen(env) == 3) {
-    s.V = (uint32_t)(env[0] - '0');
-    s.N = (uint32_t)(env[1] - '0');
-    s.Q = (uint32_t)(env[2] - '0');
-    return checked(s);
+    for (const FlatShape& x : kFlatShapes)
+      if ((int)(x.V * 100 + x.N * 10 + x.Q) == atoi(env)) return checked(x);
+    fail(RRTL_E_ARG, std::string("E_GPU_FLAT: RRTL_FLAT=") + env + " names no shape of the flat kernel");
   }
   if (explicit_w) {
     s.V = std::min(explicit_w, 4u);

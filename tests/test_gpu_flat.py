@@ -223,3 +223,18 @@ def test_more_rows_than_byte_offsets_name(engine, monkeypatch, shape):
     res = g.run(6, seed=9, stim=stim, record=rec, mode=sim.REC_HASH)
     assert g.tile_words == int(shape[0])
     assert np.array_equal(res["hash"], _ref(od, 70, 6, 9, stim, rec, 2)["hash"])
+
+
+@pytest.mark.parametrize("name", ["401", "040", "128", "412", "999", "abc"])
+def test_unknown_shapes_are_refused(wide, monkeypatch, name):
+    """A forced shape that is not built is an error of the run, not an index into the shapes' tables."""
+    cd, meta, od = wide
+    monkeypatch.setenv("RRTL_FLAT", name)
+    stim, rec = netlist_run_spec(meta)
+    g = sim.GpuBatchSimulator(cd, lanes=40)
+    with pytest.raises(sim.RrtlError) as e:
+        g.run(5, seed=1, stim=stim, record=rec, mode=sim.REC_HASH)
+    assert e.value.code == "E_GPU_FLAT"
+    monkeypatch.delenv("RRTL_FLAT")
+    res = g.run(5, seed=1, stim=stim, record=rec, mode=sim.REC_HASH)
+    assert np.array_equal(res["hash"], _ref(od, 40, 5, 1, stim, rec, 2)["hash"])
