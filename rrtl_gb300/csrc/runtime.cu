@@ -696,14 +696,22 @@ bool flat_takes(rrtl_batch* b, const rrtl_run& run) {
   return true;
 }
 
-uint32_t tuned_words(rrtl_design* d, uint32_t words) {
-  auto t = d->tuned_w.find(lane_bucket(words));
-  return t != d->tuned_w.end() && t->second != kTunedCompiled ? t->second : 0;
+// The measured choice that a batch's runs follow: a tile width,
+// kTunedCompiled, or 0 (none).
+uint32_t tuned_choice(const rrtl_batch* b) {
+  if (b->trial_words) return b->trial_words;
+  auto t = b->d->tuned_w.find(lane_bucket(b->words));
+  return t != b->d->tuned_w.end() ? t->second : 0;
+}
+
+uint32_t tuned_words(const rrtl_batch* b) {
+  const uint32_t w = tuned_choice(b);
+  return w == kTunedCompiled ? 0 : w;
 }
 
 FlatShape flat_shape_for(rrtl_batch* b, const rrtl_run& run) {
   if (!flat_takes(b, run)) return FlatShape{};
-  return choose_flat(b->d, b->words, b->tile_words, tuned_words(b->d, b->words), !b->faults.empty());
+  return choose_flat(b->d, b->words, b->tile_words, tuned_words(b), !b->faults.empty());
 }
 
 // ---- gate engine run
@@ -725,9 +733,12 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
     if (g.settle_shape.V) g.settle = flat_variant(d, g.settle_shape.V, 1, kFlatSettle);
   }
   // (the fused kernel only closes a flat run: the variant built at load time does)
-  const uint32_t W = !want_fused ? 0
-                     : g.flat    ? d->gate_w_max
-                                 : (b->tile_words ? b->tile_words : choose_tile_words(d, b->words));
+  const uint32_t trial = b->trial_words == kTunedCompiled ? 0 : b->trial_words;
+  const uint32_t W = !want_fused     ? 0
+                     : g.flat        ? d->gate_w_max
+                     : b->tile_words ? b->tile_words
+                     : trial         ? trial
+                                     : choose_tile_words(d, b->words);
   GateVariant* v = W ? gate_variant(d, W) : d->gvar[d->gate_base].get();
   const GateProgram& gp = v->gp;
   bool fused = W && v->fused_ok;
@@ -976,22 +987,23 @@ const JitKernel* fused_jit_for(rrtl_design* d, GateVariant* v) {
                        [&](JitKernel* J) { gate_fused_jit_build(v->gp, d->ctx->device, J); });
 }
 
-bool gate_jit_preferred(rrtl_design* d, uint32_t words) {
+// Whether a batch's fused-path runs should use the compiled gate kernel: the
+// autotuner's choice, else designs whose live nets fit in registers and those
+// of narrow levels.
+bool gate_jit_preferred(const rrtl_batch* b) {
+  if (b->tile_words || !b->faults.empty()) return false;
   const char* env = getenv("RRTL_GATE_JIT");
-  if (env && env[0] == '2') return true;  // A/B switch: every design within the compiled kernel's size limit
-  auto tuned = d->tuned_w.find(lane_bucket(words));
-  if (tuned != d->tuned_w.end()) return tuned->second == kTunedCompiled;
-  const GateProgram& gp = d->gp();
+  if (env && env[0] == '2' && !b->trial_words) return true;  // A/B switch: every design within its size limit
+  if (const uint32_t w = tuned_choice(b)) return w == kTunedCompiled;
+  const GateProgram& gp = b->d->gp();
   if (gp.n_real_cells > kGateJitMaxCells) return false;
   return gp.n_slots <= kGateJitAutoSlots || gp.n_real_cells < (uint64_t)kGateJitNarrowLevel * std::max(1u, gp.n_levels);
 }
 
-void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckTables* chk = nullptr,
-              bool force_compiled = false) {
+void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckTables* chk = nullptr) {
   rrtl_design* d = b->d;
   cudaStream_t st = d->ctx->stream;
-  const bool compiled = b->path == RRTL_PATH_FUSED && b->faults.empty() &&
-                        (force_compiled || (b->tile_words == 0 && gate_jit_preferred(d, b->words)));
+  const bool compiled = b->path == RRTL_PATH_FUSED && gate_jit_preferred(b);
   const FlatShape fs = b->path == RRTL_PATH_FUSED && !compiled ? flat_shape_for(b, run) : FlatShape{};
   GatePrepared g = gate_prepare(b, run, device_ptrs, b->path == RRTL_PATH_FUSED, chk, fs);
   // the compiled gate kernel: automatic tile width, no stuck-at forces; built before the timed region
@@ -1362,7 +1374,7 @@ std::vector<FlatShape> queue_shapes(rrtl_ctx* c, const std::vector<QueueJob*>& j
     rrtl_batch* b = jobs[i]->batch;
     if (!flat_takes(b, jobs[i]->run)) continue;
     const bool observe = !b->faults.empty();
-    const uint32_t base = flat_base(b->d, observe), tw = tuned_words(b->d, b->words);
+    const uint32_t base = flat_base(b->d, observe), tw = tuned_words(b);
     const FlatVariant* v = flat_variant(b->d, base, 1, observe ? kFlatObserve : kFlatPlain);
     auto add = [&](FlatShape x) {
       const double len = (double)jobs[i]->run.cycles * flat_tile_cost(v->fp, base, x);
@@ -2673,50 +2685,44 @@ rrtl_status rrtl_design_autotune(rrtl_design* d, uint32_t lanes, uint32_t cycles
     const uint32_t words = (lanes + 31) / 32;
     uint32_t best = d->gate_w_max;
     float best_t = INFINITY;
-    d->tuned_w.erase(lane_bucket(words));
-    for (uint32_t W = d->gate_w_max; W >= 1; W /= 2) {
-      if (!gate_variant(d, W)->fused_ok) continue;
+    // Each candidate is its scratch batch's alone: other batches keep the choice
+    // they have until the fastest is known, and after a failure.
+    auto time_of = [&](uint32_t choice, uint64_t n) {
       rrtl_batch* b = nullptr;
       rrtl_status st = rrtl_batch_create(d, lanes, &b);
       if (st) fail(st, g_last_error);
-      d->tuned_w[lane_bucket(words)] = W;  // as batches will run it once tuned
+      b->trial_words = choice;
       float t = INFINITY;
       try {
+        rrtl_run r = run;
+        r.cycles = n;
+        if (!flat_takes(b, r)) r.cycles = cycles;
         for (int rep = 0; rep < 3; ++rep) {
-          gate_run(b, run, false);
-          if (rep) t = std::min(t, b->last_ms);
+          gate_run(b, r, false);
+          if (rep && (choice != kTunedCompiled || b->last_tile_words == 0)) t = std::min(t, b->last_ms);
         }
       } catch (...) {
         rrtl_batch_destroy(b);
         throw;
       }
       rrtl_batch_destroy(b);
+      return t;
+    };
+    // The choice is for runs of any length, so it is made on the kernels that
+    // longer runs take: the flat kernel's shortest run where `cycles` is less.
+    const uint64_t n = std::max<uint64_t>(cycles, kFlatMinCycles);
+    auto candidate = [&](uint32_t choice) {
+      const float t = time_of(choice, n);
       if (t < best_t) {
         best_t = t;
-        best = W;
+        best = choice;
       }
-    }
+    };
+    for (uint32_t W = d->gate_w_max; W >= 1; W /= 2)
+      if (gate_variant(d, W)->fused_ok) candidate(W);
     // the compiled gate kernel, when the design qualifies
-    if (d->gp().n_real_cells <= kGateJitMaxCells) {
-      rrtl_batch* b = nullptr;
-      rrtl_status st = rrtl_batch_create(d, lanes, &b);
-      if (st) fail(st, g_last_error);
-      float t = INFINITY;
-      try {
-        for (int rep = 0; rep < 3; ++rep) {
-          gate_run(b, run, false, nullptr, true);
-          if (rep && b->last_tile_words == 0) t = std::min(t, b->last_ms);
-        }
-      } catch (...) {
-        rrtl_batch_destroy(b);
-        throw;
-      }
-      rrtl_batch_destroy(b);
-      if (t < best_t) {
-        best_t = t;
-        best = kTunedCompiled;
-      }
-    }
+    if (d->gp().n_real_cells <= kGateJitMaxCells) candidate(kTunedCompiled);
+    if (best_ms && n != cycles) best_t = time_of(best, cycles);
     d->tuned_w[lane_bucket(words)] = best;
     if (best_words) *best_words = best == kTunedCompiled ? 0u : best;
     if (best_ms) *best_ms = best_t;

@@ -186,10 +186,6 @@ WordRunDev word_chunk_desc(const WordPrepared& g, uint64_t c0, uint64_t n, bool 
 // The compiled gate kernel for this run's tables (built on first use and
 // kept per design), or nullptr when the design or run does not qualify.
 const JitKernel* gate_jit_for_run(rrtl_design* d, const GateRunTables& t, uint32_t words);
-// Whether a fused-path run of `words` 32-lane words should use the compiled
-// gate kernel: the autotuner's choice for the lane bucket, else designs whose
-// live nets fit in registers.
-bool gate_jit_preferred(rrtl_design* d, uint32_t words);
 constexpr uint32_t kTunedCompiled = 0xFFFFFFFFu;
 // Designs whose peak of live nets (the fused program's slot count) is at
 // most this use the compiled gate kernel unless tuned otherwise: beyond it
@@ -278,6 +274,7 @@ struct rrtl_batch {
   // gate engine state
   uint32_t words = 0, words_pad = 0, rows = 0;
   uint32_t tile_words = 0;  // requested fused tile width, 0 = chosen per run
+  uint32_t trial_words = 0; // the autotuner's scratch batch: the candidate it times (0: the design's choice)
   bool queued = false;      // a job of this batch is in the context's job queue
   uint32_t last_tile_words = 0;  // tile width of the last fused run, 0 after a plain run
   rrtl::DevBuf d_nets;
