@@ -41,6 +41,11 @@ void cuda_check(cudaError_t e, const char* what) {
 JobQueue::~JobQueue() {
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
+  if (fork) cudaEventDestroy(fork);
+  for (auto& e : join)
+    if (e) cudaEventDestroy(e);
+  for (auto& s : side)
+    if (s) cudaStreamDestroy(s);
 }
 
 DevBuf::~DevBuf() {
@@ -1287,6 +1292,10 @@ void word_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool start_s
 
 // ---- device job queue
 
+// Counters of a queue launch: the next item of each list; behind the fused
+// queue kernel's two, the error word of its launches.
+enum { kFusedNext = 0, kClosingNext = 2, kFlatNext = 4, kSettleNext = 5, kQueueCounters = 6 };
+
 JobQueue& queue_of(rrtl_ctx* c) {
   if (!c->queue) {
     c->queue = std::make_unique<JobQueue>();
@@ -1302,8 +1311,10 @@ void queue_finish(rrtl_ctx* c) {
   JobQueue& Q = queue_of(c);
   // launch status: a CTA that could not drain its copies fails every job of the launch
   uint32_t launch_err = 0;
-  if (Q.d_next.p && cudaMemcpy(&launch_err, Q.d_next.as<uint32_t>() + 1, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
-    launch_err = RRTL_E_DEVICE;
+  uint32_t next[kQueueCounters] = {};
+  if (Q.d_next.p && cudaMemcpy(next, Q.d_next.p, sizeof next, cudaMemcpyDeviceToHost) != cudaSuccess) launch_err = RRTL_E_DEVICE;
+  for (uint32_t e : {next[kFusedNext + 1], next[kClosingNext + 1]})
+    if (e) launch_err = e;
   std::vector<QueueJob> keep;
   for (QueueJob& j : Q.jobs) {
     if (j.status != RRTL_JOB_RUNNING) {
@@ -1432,10 +1443,10 @@ std::vector<FlatShape> queue_shapes(rrtl_ctx* c, const std::vector<QueueJob*>& j
 // One persistent launch over every queued job: each job's tiles become items
 // (all cycles of one tile), listed longest first. Jobs the flat kernel takes
 // run there, their closing settles in a second launch of it; the fused queue
-// kernel behind them runs the other jobs and the closing settles of fault
-// jobs; jobs whose recorded nets leave the chip,
-// or whose shared memory exceeds what the queue kernel can take, run on their
-// own kernels first on the same stream.
+// kernel runs the other jobs beside them and the closing settles of fault jobs
+// behind them; jobs whose recorded nets leave the chip, or whose shared memory
+// exceeds what the queue kernel can take, run on their own kernels first on
+// the same stream.
 void queue_launch(rrtl_ctx* c) {
   JobQueue& Q = queue_of(c);
   cudaStream_t st = c->stream;
@@ -1443,7 +1454,7 @@ void queue_launch(rrtl_ctx* c) {
   std::vector<GateJobDev> jobs;
   std::vector<FlatJobDev> flat_jobs;
   using Item = std::pair<double, GateItemDev>;
-  std::vector<Item> items, flat_items, settle_items;
+  std::vector<Item> items, closing_items, flat_items, settle_items;
   size_t smem = 0;
   const uint32_t launch = ++Q.launches;
   std::vector<QueueJob*> todo;
@@ -1495,9 +1506,9 @@ void queue_launch(rrtl_ctx* c) {
     const uint64_t cycles = jobs.back().R.cycles;
     const double cost = (double)(cycles + 1) * g.v->tile_cycle_cost;
     for (uint32_t t = 0; t < jobs.back().R.n_tiles; ++t)
-      items.push_back({cost, GateItemDev{ji, t, 0ull, (uint32_t)cycles, 1u}});
+      (g.flat ? closing_items : items).push_back({cost, GateItemDev{ji, t, 0ull, (uint32_t)cycles, 1u}});
   }
-  Q.last_items = (uint32_t)(items.size() + flat_items.size() + settle_items.size());
+  Q.last_items = (uint32_t)(items.size() + closing_items.size() + flat_items.size() + settle_items.size());
   auto stage = [&](std::vector<Item>& v, DevBuf& d) {
     std::stable_sort(v.begin(), v.end(), [](const Item& x, const Item& y) { return x.first > y.first; });
     std::vector<GateItemDev> flat;
@@ -1505,33 +1516,64 @@ void queue_launch(rrtl_ctx* c) {
     for (auto& it : v) flat.push_back(it.second);
     upload(d, flat);
   };
-  if (!items.empty() || !flat_items.empty()) {
-    Q.d_next.reserve(16);
-    cuda_check(cudaMemsetAsync(Q.d_next.p, 0, 16, st), "memset queue");
+  stage(items, Q.d_items);
+  stage(closing_items, Q.d_closing_items);
+  stage(flat_items, Q.d_flat_items);
+  stage(settle_items, Q.d_settle_items);
+  upload(Q.d_jobs, jobs);
+  upload(Q.d_flat_jobs, flat_jobs);
+  Q.d_next.reserve(kQueueCounters * 4);
+  cuda_check(cudaMemsetAsync(Q.d_next.p, 0, kQueueCounters * 4, st), "memset queue");
+  if (!jobs.empty() && !Q.smem_set) {
+    // the limit is per kernel: allow every job this queue can take
+    cuda_check(gate_queue_prepare(qmax), "gate_queue_prepare");
+    Q.smem_set = qmax;
   }
-  if (!flat_items.empty()) {
-    upload(Q.d_flat_jobs, flat_jobs);
-    auto run = [&](std::vector<Item>& v, DevBuf& d, uint32_t counter) {
-      if (v.empty()) return;
-      stage(v, d);
-      FlatQueueDev L{Q.d_flat_jobs.as<FlatJobDev>(), d.as<GateItemDev>(), (uint32_t)v.size(), Q.d_next.as<uint32_t>() + counter};
-      cuda_check(launch_gate_flat_queue(L, std::min<uint32_t>(L.n_items, c->sm_count), st), "gate_flat_queue_kernel");
+  const uint32_t sms = c->sm_count;
+  auto blocks = [&](const std::vector<Item>& v) { return (uint32_t)std::min<size_t>(v.size(), sms); };
+  auto fused = [&](const std::vector<Item>& v, const DevBuf& d, uint32_t counter, uint32_t grid, cudaStream_t s) {
+    if (!grid) return;
+    GateQueueDev QD{Q.d_jobs.as<GateJobDev>(), d.as<GateItemDev>(), (uint32_t)v.size(), Q.d_next.as<uint32_t>() + counter};
+    cuda_check(launch_gate_queue(QD, grid, smem, s), "gate_queue_kernel");
+  };
+  auto flat = [&](const std::vector<Item>& v, const DevBuf& d, uint32_t counter) {
+    if (v.empty()) return;
+    FlatQueueDev L{Q.d_flat_jobs.as<FlatJobDev>(), d.as<GateItemDev>(), (uint32_t)v.size(), Q.d_next.as<uint32_t>() + counter};
+    cuda_check(launch_gate_flat_queue(L, blocks(v), st), "gate_flat_queue_kernel");
+  };
+  if (!items.empty() && !flat_items.empty()) {
+    // Both lists at once: a block of either kernel fills an SM, so the fused
+    // kernel first gets at most half of them (more where the flat list is
+    // short), the flat one all it finds, and the fused one's other blocks
+    // follow as SMs come free: both start with their longest items and no SM
+    // waits for the other list's last one.
+    struct Joins {
+      JobQueue& Q;
+      cudaStream_t st;
+      ~Joins() {  // (also when a later launch fails)
+        for (auto& e : Q.join) cudaStreamWaitEvent(st, e, 0);
+      }
     };
-    run(flat_items, Q.d_flat_items, 2);
-    run(settle_items, Q.d_settle_items, 3);
+    for (auto& s : Q.side)
+      if (!s) cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
+    for (cudaEvent_t* e : {&Q.fork, &Q.join[0], &Q.join[1]})
+      if (!*e) cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "event");
+    const uint32_t all = blocks(items), first = std::min(all, std::max(sms / 2, sms - blocks(flat_items)));
+    cuda_check(cudaEventRecord(Q.fork, st), "event");
+    for (auto& s : Q.side) cuda_check(cudaStreamWaitEvent(s, Q.fork, 0), "event");
+    Joins joins{Q, st};
+    fused(items, Q.d_items, kFusedNext, first, Q.side[0]);
+    cuda_check(cudaEventRecord(Q.join[0], Q.side[0]), "event");
+    flat(flat_items, Q.d_flat_items, kFlatNext);
+    fused(items, Q.d_items, kFusedNext, all - first, Q.side[1]);
+    cuda_check(cudaEventRecord(Q.join[1], Q.side[1]), "event");
+    flat(settle_items, Q.d_settle_items, kSettleNext);
+  } else {
+    fused(items, Q.d_items, kFusedNext, blocks(items), st);
+    flat(flat_items, Q.d_flat_items, kFlatNext);
+    flat(settle_items, Q.d_settle_items, kSettleNext);
   }
-  if (!items.empty()) {
-    stage(items, Q.d_items);
-    upload(Q.d_jobs, jobs);
-    if (!Q.smem_set) {
-      // the limit is per kernel: allow every job this queue can take
-      cuda_check(gate_queue_prepare(qmax), "gate_queue_prepare");
-      Q.smem_set = qmax;
-    }
-    GateQueueDev QD{Q.d_jobs.as<GateJobDev>(), Q.d_items.as<GateItemDev>(), (uint32_t)items.size(), Q.d_next.as<uint32_t>()};
-    const uint32_t grid = std::min<uint32_t>((uint32_t)items.size(), c->sm_count);
-    cuda_check(launch_gate_queue(QD, grid, smem, st), "gate_queue_kernel");
-  }
+  fused(closing_items, Q.d_closing_items, kClosingNext, blocks(closing_items), st);
   cuda_check(cudaEventRecord(Q.ev1, st), "event");
 }
 

@@ -151,7 +151,10 @@ struct JobQueue {
   uint32_t launches = 0;
   std::vector<QueueJob> jobs;                 // queued or running
   std::unordered_map<uint64_t, uint32_t> finished;  // id -> RRTL_JOB_DONE / RRTL_JOB_FAILED
-  DevBuf d_jobs, d_items, d_next, d_flat_jobs, d_flat_items, d_settle_items;
+  DevBuf d_jobs, d_items, d_closing_items, d_next, d_flat_jobs, d_flat_items, d_settle_items;
+  // launches beside the flat queue kernel (created on the first mixed launch)
+  cudaStream_t side[2] = {};
+  cudaEvent_t fork = nullptr, join[2] = {};
   size_t smem_set = 0;                        // dynamic shared memory the queue kernel is prepared for
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;   // around the last launch
   float last_ms = 0.f;
