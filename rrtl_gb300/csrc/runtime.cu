@@ -720,6 +720,38 @@ FlatShape flat_shape_for(rrtl_batch* b, const rrtl_run& run) {
 }
 
 // ---- gate engine run
+// Validate a run and list its stimulus and record tables (without slots).
+GateRunTables gate_tables(rrtl_batch* b, const rrtl_run& run, const CheckTables* chk) {
+  rrtl_design* d = b->d;
+  const GateProgram& gp = d->gp();  // nets are the same in every variant
+  GateRunTables t;
+  for (uint32_t i = 0; i < run.n_stim; ++i) {
+    const rrtl_stim& s = run.stim[i];
+    signal_of(d, s.signal);
+    uint32_t net = gp.signal_net[s.signal];
+    REQUIRE(gp.net_is_source[net], RRTL_E_ARG, "E_GPU_STIM: stimulus targets a combinationally driven signal");
+    REQUIRE(s.kind <= RRTL_STIM_RANDOM_UNIFORM, RRTL_E_ARG, "E_GPU_STIM: unknown stimulus kind");
+    if (s.kind == RRTL_STIM_TRACE)
+      REQUIRE(s.param < run.n_trace_cols && run.input_trace, RRTL_E_ARG, "E_GPU_STIM: trace column out of range");
+    t.stim.push_back(GateStimDev{0u, net, s.kind, 0, s.param});
+  }
+  for (uint32_t i = 0; i < run.n_record; ++i) {
+    signal_of(d, run.record[i]);
+    t.rec.push_back(GateRecDev{0u, gp.signal_net[run.record[i]]});
+  }
+  t.mode = run.record_mode;
+  REQUIRE(!(t.mode & (RRTL_REC_TRACE | RRTL_REC_HASH | RRTL_REC_DETECT)) || run.n_record > 0, RRTL_E_ARG,
+          "E_GPU_RECORD: recording needs at least one signal");
+  REQUIRE(run.cycles < (1ull << 32), RRTL_E_ARG, "E_GPU_STEPS: cycle count exceeds 2^32");
+  REQUIRE(run.lane_base % 32 == 0 && run.lane_base < (1ull << 40), RRTL_E_ARG,
+          "E_GPU_LANE_BASE: lane_base must be a multiple of 32 below 2^40");
+  REQUIRE(!(t.mode & RRTL_REC_CHECK) || chk, RRTL_E_ARG, "E_GPU_RECORD: checks are for trace replay");
+  REQUIRE(!(t.mode & RRTL_REC_TRACE) || run.out_trace, RRTL_E_ARG, "E_GPU_RECORD: out_trace is null");
+  REQUIRE(!(t.mode & RRTL_REC_HASH) || run.out_hash, RRTL_E_ARG, "E_GPU_RECORD: out_hash is null");
+  REQUIRE(!(t.mode & RRTL_REC_DETECT) || run.detect, RRTL_E_ARG, "E_GPU_RECORD: detect is null");
+  return t;
+}
+
 // Validate a run, pick the program variant and upload its stimulus and record
 // tables; stages host input traces and zeroes hash/detect outputs on the
 // context stream. `want_fused` asks for the fused path (it falls back to the
@@ -747,24 +779,11 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   GateVariant* v = W ? gate_variant(d, W) : d->gvar[d->gate_base].get();
   const GateProgram& gp = v->gp;
   bool fused = W && v->fused_ok;
-  std::vector<GateStimDev> stim;
-  for (uint32_t i = 0; i < run.n_stim; ++i) {
-    const rrtl_stim& s = run.stim[i];
-    signal_of(d, s.signal);
-    uint32_t net = gp.signal_net[s.signal];
-    REQUIRE(gp.net_is_source[net], RRTL_E_ARG, "E_GPU_STIM: stimulus targets a combinationally driven signal");
-    REQUIRE(s.kind <= RRTL_STIM_RANDOM_UNIFORM, RRTL_E_ARG, "E_GPU_STIM: unknown stimulus kind");
-    if (s.kind == RRTL_STIM_TRACE)
-      REQUIRE(s.param < run.n_trace_cols && run.input_trace, RRTL_E_ARG, "E_GPU_STIM: trace column out of range");
-    stim.push_back(GateStimDev{0u, net, s.kind, 0, s.param});
-  }
-  std::vector<GateRecDev> rec;
-  for (uint32_t i = 0; i < run.n_record; ++i) {
-    signal_of(d, run.record[i]);
-    uint32_t net = gp.signal_net[run.record[i]];
-    if (fused && !g.flat && !v->end_live[net]) fused = false;  // value not held to the end of the cycle: use the plain path
-    rec.push_back(GateRecDev{0u, net});
-  }
+  g.tables = gate_tables(b, run, chk);
+  std::vector<GateStimDev>& stim = g.tables.stim;
+  std::vector<GateRecDev>& rec = g.tables.rec;
+  for (const GateRecDev& r : rec)
+    if (!g.flat && !v->end_live[r.net]) fused = false;  // value not held to the end of the cycle: use the plain path
   if (fused) {
     const std::vector<int32_t>& rows = g.flat ? g.flat->fp.net_slot : gp.net_slot;
     for (auto& r : rec) r.slot = (uint32_t)rows[r.net];
@@ -774,14 +793,8 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
         for (auto& s : stim)
           if (r.net == s.net) g.R.flat_serial = 1;
   }
-  REQUIRE(!(run.record_mode & (RRTL_REC_TRACE | RRTL_REC_HASH | RRTL_REC_DETECT)) || run.n_record > 0, RRTL_E_ARG,
-          "E_GPU_RECORD: recording needs at least one signal");
-  REQUIRE(run.cycles < (1ull << 32), RRTL_E_ARG, "E_GPU_STEPS: cycle count exceeds 2^32");
   upload(b->d_stim, stim);
   upload(b->d_rec, rec);
-  g.tables.stim = stim;
-  g.tables.rec = rec;
-  g.tables.mode = run.record_mode;
 
   GateRunDev& R = g.R;
   R.cycles = run.cycles;
@@ -812,10 +825,7 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   R.nets = b->d_nets.as<uint32_t>();
   R.err = b->d_err.as<uint32_t>();
   R.cycle_base = 0;
-  REQUIRE(run.lane_base % 32 == 0 && run.lane_base < (1ull << 40), RRTL_E_ARG,
-          "E_GPU_LANE_BASE: lane_base must be a multiple of 32 below 2^40");
   R.word_base = run.lane_base / 32;
-  REQUIRE(!(run.record_mode & RRTL_REC_CHECK) || chk, RRTL_E_ARG, "E_GPU_RECORD: checks are for trace replay");
   if (chk) {
     R.chk_idx = chk->idx;
     R.chk_exp = chk->exp;
@@ -830,9 +840,6 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   g.want_trace = run.record_mode & RRTL_REC_TRACE;
   g.want_hash = run.record_mode & RRTL_REC_HASH;
   g.want_det = run.record_mode & RRTL_REC_DETECT;
-  REQUIRE(!g.want_trace || run.out_trace, RRTL_E_ARG, "E_GPU_RECORD: out_trace is null");
-  REQUIRE(!g.want_hash || run.out_hash, RRTL_E_ARG, "E_GPU_RECORD: out_hash is null");
-  REQUIRE(!g.want_det || run.detect, RRTL_E_ARG, "E_GPU_RECORD: detect is null");
   if (device_ptrs) {
     R.in_trace = run.input_trace;
     R.out_trace = run.out_trace;
@@ -1008,11 +1015,15 @@ bool gate_jit_preferred(const rrtl_batch* b) {
 void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckTables* chk = nullptr) {
   rrtl_design* d = b->d;
   cudaStream_t st = d->ctx->stream;
-  const bool compiled = b->path == RRTL_PATH_FUSED && gate_jit_preferred(b);
-  const FlatShape fs = b->path == RRTL_PATH_FUSED && !compiled ? flat_shape_for(b, run) : FlatShape{};
-  GatePrepared g = gate_prepare(b, run, device_ptrs, b->path == RRTL_PATH_FUSED, chk, fs);
+  const bool on_chip = b->path == RRTL_PATH_FUSED;
   // the compiled gate kernel: automatic tile width, no stuck-at forces; built before the timed region
-  const JitKernel* J = compiled && !g.R.has_forces ? gate_jit_for_run(d, g.tables, b->words) : nullptr;
+  const JitKernel* J = on_chip && gate_jit_preferred(b) ? gate_jit_for_run(d, gate_tables(b, run, chk), b->words) : nullptr;
+  // Without it (too many entries, not built, another thread builds it) the run
+  // goes where other designs' runs go. us a cycle of designs that prefer it,
+  // flat / fused kernel: crc32 2.1 / 4.8 at 64 lanes, 16.6 / 34.0 at 262,144;
+  // 32-bit ALU planes 7.5 / 64.9 and 82.8 / 465.
+  const FlatShape fs = on_chip && !J ? flat_shape_for(b, run) : FlatShape{};
+  GatePrepared g = gate_prepare(b, run, device_ptrs, on_chip, chk, fs);
   // the fused kernel compiled for the design's truth-table classes, also built before the timed region
   // (not for a settle alone, which runs the same code in both)
   const JitKernel* F = !J && g.fused && !g.flat && run.cycles ? fused_jit_for(d, g.v) : nullptr;
