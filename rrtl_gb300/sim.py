@@ -58,6 +58,15 @@ _STIM_DTYPE = np.dtype([("signal", np.uint32), ("kind", np.uint32), ("param", np
 assert _STIM_DTYPE.itemsize == ctypes.sizeof(Stim)
 
 
+def _wrapped(values, dtype) -> np.ndarray:
+    """Integers (NumPy scalars too) reduced to the width of `dtype`, as a field of a C structure takes them."""
+    v = list(map(operator.index, values))
+    try:
+        return np.array(v, dtype=dtype)
+    except OverflowError:
+        return np.array([x & ((1 << 8 * dtype.itemsize) - 1) for x in v], dtype=dtype)
+
+
 class Run(ctypes.Structure):
     _fields_ = [
         ("cycles", c_uint64),
@@ -509,17 +518,21 @@ class CompiledDesign:
             self._engine = self.info.engine
         return self._engine
 
-    def index(self, s) -> int:
-        """Packed index of a signal given by name (or index)."""
-        if isinstance(s, str):
-            return (self._cache.get(s) or self.signal(s))[0]
-        if isinstance(s, int):
-            return s
-        raise TypeError("signals are addressed by name or packed index")
-
     def indices(self, signals) -> np.ndarray:
         """Packed indices of signals given by name (or index); OverflowError for an index outside 32 bits."""
-        return np.array([self.index(s) for s in signals], dtype=np.uint32)
+        return np.array(self._index_list(signals), dtype=np.uint32)
+
+    def _index_list(self, signals) -> list:
+        cache = self._cache
+        out = []
+        for s in signals:
+            if isinstance(s, str):
+                out.append((cache.get(s) or self.signal(s))[0])
+            elif isinstance(s, int):
+                out.append(s)
+            else:
+                raise TypeError("signals are addressed by name or packed index")
+        return out
 
     def signal(self, name: str):
         """(index, width, kind) of a signal by name."""
@@ -730,10 +743,12 @@ class GpuBatchSimulator:
     def make_run(self, cycles: int, seed: int = 0, stim: Iterable = (), record: Iterable = (), mode: int = 0,
                  input_trace: Optional[np.ndarray] = None, out_trace=None, out_hash=None, detect=None,
                  lane_base: int = 0) -> Run:
-        # any integer (a NumPy scalar too), reduced to its field's width as a C structure takes it
-        st = [(self.design.index(s) & 0xFFFFFFFF, operator.index(k) & 0xFFFFFFFF, operator.index(p) & 0xFFFFFFFFFFFFFFFF)
-              for s, k, p in stim]
-        arr = np.array(st or [(0, 0, 0)], dtype=_STIM_DTYPE)
+        st = [(s, k, p) for s, k, p in stim]
+        arr = np.zeros(max(1, len(st)), dtype=_STIM_DTYPE)
+        if st:
+            names, kinds, params = zip(*st)
+            for field, values in (("signal", self.design._index_list(names)), ("kind", kinds), ("param", params)):
+                arr[field] = _wrapped(values, _STIM_DTYPE[field])
         rec = self.design.indices(record)
         r = Run()
         r.cycles = cycles
