@@ -431,18 +431,19 @@ uint32_t choose_tile_words(rrtl_design* d, uint32_t words) {
 // explicit tile width. RRTL_FLAT=0 keeps the fused kernel and RRTL_FLAT=VNQ
 // forces a shape (A/B switches).
 //
-// The cost of a tile-cycle in SM clocks was fitted to one wave of tiles on
-// netlists of 41 levels and 10,000 / 50,000 / 200,000 gates for narrow tiles:
-// one word 12.1k / 24.6k / 66.9k (24 warps 12.1k / 23.7k / 59.1k), two 13.8k /
-// 28.7k / 80.9k (13.8k / 28.0k / 74.3k); and on 3,000 / 10,000 / 20,000 /
-// 50,000 gates: one 4-word vector 12.9k / 17.4k / 22.7k
-// / 37.2k, two 16.4k / 24.8k / 33.5k / 56.1k, four as two warp sets of two
-// 24.8k / 36.9k / 53.9k / 97.8k (sets of one vector: four sets 25.3k / 37.1k
-// / 57.3k / 114k, two sets against two vectors 17.8k / 24.8k / 35.6k /
-// 62.5k). So a tile costs about 220 clocks a level and 9 an entry, and each
-// vector one a wavefront and 75 a level; wide tiles pay until SMs are left
-// without one. (A one-word tile in the queue is priced above its 20.3 clocks an
-// entry: at that price a stream of 24 jobs took 11.5 instead of 11.0 ms.)
+// A tile-cycle costs a boundary (stimulus, record, two barriers), a part per
+// level, one per entry and, in wide tiles, one per vector and its wavefronts.
+// Clocks, fitted to one wave of tiles on ten netlists of 3,000 to 200,000 gates
+// and 11 to 158 levels; the fit is within 8% of every one- and two-word tile
+// and 11% of every wider one (without the boundary: 41%, too low at 11 levels).
+// Measured, clocks a tile-cycle at 10,000 gates and 11 / 41 / 155 levels and at
+// 50,000 and 200,000 gates and 41 levels: one word 7.4k / 12.1k / 34.8k / 23.4k /
+// 58.9k (in the queue, 16 warps: 7.4k / 11.8k / 34.1k / 24.9k / 66.9k), two
+// 9.1k / 13.7k / 36.9k / 27.9k / 74.3k (8.9k / 13.7k / 36.7k / 29.3k / 80.9k),
+// one 4-word vector 10.9k / 17.5k / 44.5k / 36.6k / 105k, two 16.1k / 25.2k /
+// 56.8k / 56.2k, three 21.2k / 32.5k / 77.1k / 76.5k, four as two warp sets of
+// two 22.0k / 36.9k / 77.9k / 95.8k. Wide tiles pay until SMs are left without
+// one.
 constexpr FlatShape kFlatShapes[] = {{4, 2, 2}, {4, 3, 1}, {4, 2, 1}, {4, 1, 1}, {2, 1, 1}, {1, 1, 1}};
 // The tile width a flat run reports: several tiles of the widest documented
 // width that divides its own.
@@ -452,9 +453,10 @@ uint32_t flat_reported_words(uint32_t w) { return w == 16 ? 8 : w == 12 ? 4 : w;
 // width `base`.
 double flat_tile_cost(const FlatProgram& fp, uint32_t base, const FlatShape& x) {
   const double L = fp.n_levels, E = fp.n_entries;
-  if (x.V != 4) return 173.0 * L + (x.V == 2 ? (x.narrow ? 23.0 : 25.0) : x.narrow ? 18.5 : 21.7) * E;
+  if (x.V == 1) return x.narrow ? 3060.0 + 162.0 * L + 15.1 * E : 2880.0 + 147.0 * L + 17.4 * E;
+  if (x.V == 2) return x.narrow ? 3800.0 + 157.0 * L + 19.7 * E : 3550.0 + 159.0 * L + 21.2 * E;
   const double vec4 = (double)fp.wavefronts * (base == 4 ? 1.0 : base == 2 ? 1.9 : 3.6);  // wavefronts of 4-word rows
-  return 222.0 * L + 9.1 * E + x.N * x.Q * (1.03 * vec4 + 75.0 * L);
+  return 3280.0 + 158.0 * L + 8.3 * E + x.N * x.Q * (935.0 + 49.0 * L + 1.06 * vec4);
 }
 
 // The widest rows that fit (0: none); packing leaves fewer live nets than the
@@ -469,7 +471,7 @@ bool flat_fits(rrtl_design* d, const FlatShape& x, bool observe) {
   return flat_variant(d, x.V, x.Q, x.narrow ? kFlatNarrow : observe ? kFlatObserve : kFlatPlain)->max_n >= x.N * x.Q;
 }
 
-FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w, uint32_t tuned_w, bool observe) {
+FlatShape choose_flat(rrtl_design* d, uint32_t words, uint64_t cycles, uint32_t explicit_w, uint32_t tuned_w, bool observe) {
   FlatShape s;
   auto checked = [&](FlatShape x) {
     x.narrow = x.V < 4 && !observe;
@@ -496,8 +498,12 @@ FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w, uint3
     x.narrow = x.V < 4 && !observe;
     if (x.V > top || (x.V == 4 && x.N * x.Q > v->max_n)) continue;
     if (tuned_w && flat_reported_words(x.words()) != tuned_w) continue;
-    // (tiles past one a SM are split between blocks: no last round)
-    const double t = std::max(1.0, std::ceil((double)words / x.words()) / d->ctx->sm_count) * flat_tile_cost(v->fp, top, x);
+    // Tiles past one a SM are split between blocks: no last round, but a split
+    // tile is loaded and stored once more, up to two tile-cycles a run (172
+    // one-word tiles on 152 SMs: 1.1 to 2.4 on the netlists above).
+    const uint32_t tiles = (words + x.words() - 1) / x.words(), sms = d->ctx->sm_count;
+    const double split = tiles > sms && tiles % sms ? 2.0 / (double)cycles : 0.0;
+    const double t = (std::max(1.0, (double)tiles / sms) + split) * flat_tile_cost(v->fp, top, x);
     if (t < best) {
       best = t;
       s = x;
@@ -506,9 +512,12 @@ FlatShape choose_flat(rrtl_design* d, uint32_t words, uint32_t explicit_w, uint3
   return checked(s);
 }
 
-// Shape of a closing settle over `words` words (V = 0: none fits), by the cost
-// of one tile-cycle of the cycles' program: its settle has the unpacked cells
-// (1.3 times the entries), the same for every shape.
+// Shape of a closing settle over `words` words (V = 0: none fits), by rounds
+// times the cost of a tile-cycle with its program's levels, entries and
+// wavefronts. At 7 to 3,000 words of netlists of 2,000 to 200,000 gates and 11
+// to 161 levels it chose the fastest of the four shapes, or one within 6% (us at
+// 50,000 gates, one word / two / one 4-word vector / two: 52 / 56 / 64 / 106 at
+// 7 words, 195 / 135 / 76 / 134 at 313, 1,076 / 606 / 434 / 397 at 3,000).
 FlatShape choose_settle(rrtl_design* d, uint32_t words) {
   FlatShape s;
   uint32_t top = 0;
@@ -716,7 +725,7 @@ uint32_t tuned_words(const rrtl_batch* b) {
 
 FlatShape flat_shape_for(rrtl_batch* b, const rrtl_run& run) {
   if (!flat_takes(b, run)) return FlatShape{};
-  return choose_flat(b->d, b->words, b->tile_words, tuned_words(b), !b->faults.empty());
+  return choose_flat(b->d, b->words, run.cycles, b->tile_words, tuned_words(b), !b->faults.empty());
 }
 
 // ---- gate engine run
