@@ -766,7 +766,7 @@ GateRunTables gate_tables(rrtl_batch* b, const rrtl_run& run, const CheckTables*
 // context stream. `want_fused` asks for the fused path (it falls back to the
 // plain path when a recorded net does not stay on chip to the end of a cycle).
 GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool want_fused,
-                          const CheckTables* chk, FlatShape flat) {
+                          const CheckTables* chk, FlatShape flat, GateRunTables* tables) {
   rrtl_design* d = b->d;
   cudaStream_t st = d->ctx->stream;
   GatePrepared g;
@@ -788,7 +788,7 @@ GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, 
   GateVariant* v = W ? gate_variant(d, W) : d->gvar[d->gate_base].get();
   const GateProgram& gp = v->gp;
   bool fused = W && v->fused_ok;
-  g.tables = gate_tables(b, run, chk);
+  g.tables = tables ? std::move(*tables) : gate_tables(b, run, chk);
   std::vector<GateStimDev>& stim = g.tables.stim;
   std::vector<GateRecDev>& rec = g.tables.rec;
   for (const GateRecDev& r : rec)
@@ -1026,13 +1026,14 @@ void gate_run(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, const CheckT
   cudaStream_t st = d->ctx->stream;
   const bool on_chip = b->path == RRTL_PATH_FUSED;
   // the compiled gate kernel: automatic tile width, no stuck-at forces; built before the timed region
-  const JitKernel* J = on_chip && gate_jit_preferred(b) ? gate_jit_for_run(d, gate_tables(b, run, chk), b->words) : nullptr;
+  GateRunTables tables = gate_tables(b, run, chk);
+  const JitKernel* J = on_chip && gate_jit_preferred(b) ? gate_jit_for_run(d, tables, b->words) : nullptr;
   // Without it (too many entries, not built, another thread builds it) the run
   // goes where other designs' runs go. us a cycle of designs that prefer it,
   // flat / fused kernel: crc32 2.1 / 4.8 at 64 lanes, 16.6 / 34.0 at 262,144;
   // 32-bit ALU planes 7.5 / 64.9 and 82.8 / 465.
   const FlatShape fs = on_chip && !J ? flat_shape_for(b, run) : FlatShape{};
-  GatePrepared g = gate_prepare(b, run, device_ptrs, on_chip, chk, fs);
+  GatePrepared g = gate_prepare(b, run, device_ptrs, on_chip, chk, fs, &tables);
   // the fused kernel compiled for the design's truth-table classes, also built before the timed region
   // (not for a settle alone, which runs the same code in both)
   const JitKernel* F = !J && g.fused && !g.flat && run.cycles ? fused_jit_for(d, g.v) : nullptr;

@@ -171,8 +171,9 @@ struct CheckTables {
 };
 
 // Runtime internals shared by the C ABI and the serving loop.
+// (tables: the run's, where the caller has listed them already)
 GatePrepared gate_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool want_fused,
-                          const CheckTables* chk = nullptr, FlatShape flat = FlatShape{});
+                          const CheckTables* chk = nullptr, FlatShape flat = FlatShape{}, GateRunTables* tables = nullptr);
 void gate_copy_out(rrtl_batch* b, const GatePrepared& g, const rrtl_run& run);
 void gate_plain_launches(const GatePrepared& g, uint64_t cycles, cudaStream_t st, bool graph);
 WordPrepared word_prepare(rrtl_batch* b, const rrtl_run& run, bool device_ptrs, bool start_settle,
