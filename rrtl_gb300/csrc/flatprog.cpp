@@ -949,8 +949,6 @@ FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOpti
     if (made[n] >= 0 && last[n] >= kEnd) fp.recordable[n] = 1;
     if (gp.net_is_source[n] && !is_q[n]) fp.recordable[n] = 1;
   }
-  for (uint32_t i = 0; i < cells.size(); ++i)
-    if (lg.alive[i]) fp.cells.push_back(cells[i]);
   return fp;
 }
 

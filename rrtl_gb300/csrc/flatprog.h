@@ -34,7 +34,6 @@
 
 namespace rrtl {
 
-
 // One lane of a stream entry.
 //  two cells of two inputs: x = a | b << 16, y = out | meta; z, w the second
 //  one cell of three inputs (kFlatDevThree): x = a | b << 16, y = out | meta,
@@ -60,7 +59,6 @@ struct FlatCell {
 struct FlatProgram {
   uint32_t V = 4, G = 8;
   uint32_t warps = 16;                    // streams: warps of the set that walks the program
-  std::vector<FlatCell> cells;            // packed cells, by level
   uint32_t n_levels = 0;
   std::vector<int32_t> net_slot;          // -1: not resident
   std::vector<uint8_t> recordable;        // net holds its value in its slot when the cycle's settle ends
@@ -79,7 +77,7 @@ struct FlatProgram {
 };
 
 struct FlatOptions {
-  bool pack = true;
+  bool pack = true;       // (false: only for the CPU tests of the other parts, as below)
   bool fold_regs = true;
   bool settle = false;   // a closing settle: every signal computed and written back, no registers committed
   bool observe = false;  // every signal keeps a row of its own (stuck-at forces act on any of them)

@@ -24,16 +24,16 @@ __device__ __forceinline__ bool flat_wait_part(const uint32_t* done, uint64_t cy
   return __syncthreads_and(ok);
 }
 
+template <int V, bool F>
+constexpr uint32_t flat_compute_threads() { return V < 4 && !F ? kFlatNarrowThreads : kFlatComputeThreads; }
+
 // Blocks take equal shares of the run (flat_part) where its tiles do not fill
 // the last round. A split tile costs one more load and store of its sources
-// (about a cycle), a last round up to all of the run: 200,000 gates, 10,007
+// (one to two cycles), a last round up to all of the run: 200,000 gates, 10,007
 // lanes x 100 cycles (157 tiles of 2 words on 152 SMs) 6.35 -> 5.36 ms; 50,000
 // gates, 5,003 x 200 (157 of 1) 3.11 -> 2.91. At 65,536 lanes x 1,000 it makes
 // 171 tiles of 12 words (42.5 ms) better than 128 of 16 (47.0), which leave 24
 // SMs without a tile.
-template <int V, bool F>
-constexpr uint32_t flat_compute_threads() { return V < 4 && !F ? kFlatNarrowThreads : kFlatComputeThreads; }
-
 template <int V, int N, int Q, bool F, bool kFull, bool kBytes>
 __global__ void __launch_bounds__(flat_compute_threads<V, F>() + kFlatServiceThreads, 1) gate_flat_kernel(FlatProgDev P, GateRunDev R) {
   extern __shared__ __align__(128) uint8_t smem[];

@@ -363,6 +363,9 @@ FlatVariant* flat_variant(rrtl_design* d, uint32_t V, uint32_t Q, FlatKind kind)
     P.n_slots = fp.n_slots;
     P.warps = fp.warps;
   }
+  // on the device, or not used: a design keeps what runs are prepared from
+  for (auto* s : {&v->fp.stream_net, &v->fp.source_nets}) std::vector<uint32_t>().swap(*s);
+  std::vector<FlatLane>().swap(v->fp.stream);
   slot = std::move(v);
   return slot.get();
 }
