@@ -759,7 +759,8 @@ def crc32_leg(ctx, sim, cycles=2000):
     256K / 1M lanes). Random din per lane per cycle, reset on cycle 0; the
     compiled gate kernel with no per-cycle recording (state only, like the
     reference's run) and with a per-cycle hash of the 32 crc outputs, the
-    fused kernel (tile width 8) beside it; per-cycle hashes compared."""
+    flat gate kernel (tile width 8; the "fused_hash" rows) beside it; per-cycle
+    hashes compared."""
     cd = sim.CompiledDesign(crc32_netlist(), "crc32", ctx)
     stim = [("clk", sim.STIM_CONST, 1), ("rst", sim.STIM_PULSE, 1)] + [(f"din_{i}", sim.STIM_RANDOM, i) for i in range(8)]
     rec = [f"crc_{i}" for i in range(32)]
@@ -1098,8 +1099,8 @@ def main():
     achieved = algo_bytes / (ms_step / 1000.0) / 1e9
     # the roof that binds: every cell-word evaluation reads its fanin rows and
     # writes its output row in shared memory, so the net-streaming bytes are
-    # the kernel's shared-memory traffic; the nominal shared-memory bandwidth
-    # is 128 bytes per clock per SM
+    # the kernel's shared-memory traffic (more than the packed cells move); the
+    # nominal shared-memory bandwidth is 128 bytes per clock per SM
     sm_mhz = clock_summary.get("sm_mhz") or 2070.0
     smem_peak = ctx.sm_count * 128.0 * sm_mhz * 1e6 / 1e9
     issue = profiled_issue("gate_flat_kernel_c2.md")
@@ -1108,19 +1109,18 @@ def main():
     traffic, tlanes = profiled_traffic("gate_flat_kernel_c2.md")
     if traffic is not None:
         traffic = traffic * LANES / tlanes
-    roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": traffic, "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
-                else "fallback", "bytes_per_lane_cycle": bpl,
+    roofline = {"bound": "smem", "achieved": achieved, "peak": smem_peak, "unit": "GB/s", "frac": achieved / smem_peak,
+                "traffic": traffic, "peak_kind": f"nominal: {ctx.sm_count} SMs x 128 B/clock x {sm_mhz:.0f} MHz (sampled "
+                                                 f"SM clock)", "bytes_per_lane_cycle": bpl,
                 "model": "net-streaming bytes per lane-cycle (fanin reads + output write per gate, D read + Q write "
-                         "per flop, inputs and outputs), 4 bytes per 32 lanes",
-                "note": "nets stay in shared memory for all cycles of a tile, so measured DRAM traffic per launch "
-                        "(traffic) is far below the streamed bytes (achieved*time): HBM does not bind this kernel; "
-                        "the shared-memory roof below does",
-                "smem": {"bound": "smem", "achieved": achieved, "peak": smem_peak, "unit": "GB/s",
-                         "frac": achieved / smem_peak,
-                         "peak_kind": f"nominal: {ctx.sm_count} SMs x 128 B/clock x {sm_mhz:.0f} MHz (sampled SM clock)",
-                         "model": "the net-streaming bytes are the cell evaluations' shared-memory row reads and "
-                                  "writes"},
+                         "per flop, inputs and outputs), 4 bytes per 32 lanes: the cell evaluations' shared-memory row "
+                         "reads and writes",
+                "hbm": {"achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                        "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
+                        else "fallback",
+                        "note": "the same bytes against the copy bandwidth, for scale: nets stay in shared memory for "
+                                "all cycles of a tile, so measured DRAM traffic per launch (traffic) is far below the "
+                                "streamed bytes (achieved*time) and HBM does not bind this kernel"},
                 "issue": issue}
     out = {
         "metric": METRIC, "value": value, "unit": "lane-cycles/s", "n_gpus": ws, "steps": args.steps,
