@@ -289,7 +289,9 @@ rrtl_status rrtl_batch_set_tile_words(rrtl_batch* b, uint32_t words);
  * 2712-2721, re-aimed at this engine's knob): times `cycles` cycles of a
  * scratch batch of `lanes` lanes at every tile width that fits and makes the
  * fastest the choice for batches of that size (same power-of-two bucket of
- * 32-lane words). Gate engine; the word engine has no width and reports 0. */
+ * 32-lane words; for fewer than four cycles the choice is made over four,
+ * which run on another kernel than fewer do). A failed call leaves the choice
+ * as it was. Gate engine; the word engine has no width and reports 0. */
 rrtl_status rrtl_design_autotune(rrtl_design* design, uint32_t lanes, uint32_t cycles, uint32_t* best_words,
                                  float* best_ms);
 rrtl_status rrtl_batch_tile_words(rrtl_batch* b, uint32_t* words);
@@ -539,11 +541,13 @@ enum { RRTL_JIT_SPLIT = 1 };
  * compiled for the design and the run's tables: one thread per 32-lane word,
  * every net a register, one LOP3 per cell (the reference's per-design
  * compiled kernel, crates/rrtl-sim-ir/src/gpu_codegen.rs:503-557). Designs
- * whose live nets fit in registers (at most 192 at once) use it unless the
- * autotuner measured a tile width faster for the lane count (larger designs
- * spill and run faster on the fused kernel); rrtl_design_autotune times it as a candidate and
- * reports it as best_words = 0. rrtl_batch_tile_words reads 0 after such a
- * run. This call emits (and with arch compiles) that kernel without a device,
+ * whose live nets fit in registers (at most 192 at once) or whose levels are
+ * narrow use it unless the autotuner measured a tile width faster for the lane
+ * count (compiling it for a larger design takes seconds); rrtl_design_autotune
+ * times it as a candidate and reports it as best_words = 0.
+ * rrtl_batch_tile_words reads 0 after such a run. A run of more than 64
+ * stimulus or record entries, or one whose kernel is not built, takes the flat
+ * gate kernel instead. This call emits (and with arch compiles) that kernel without a device,
  * like rrtl_word_jit_emit; run is required (its signals are packed indices).
  * RRTL_E_UNSUPPORTED when the design is outside the gate engine. */
 rrtl_status rrtl_gate_jit_emit(const char* json, size_t len, const char* top, const rrtl_run* run, const char* arch,

@@ -8,8 +8,8 @@
 // C++: one thread per 32-lane word for all cycles, every net a register, one
 // LOP3 per cell in level order and the register commit unrolled; the random
 // or traced stimulus and the record stage run on other warps of its block. It serves runs without stuck-at
-// forces on designs of up to kGateJitMaxCells cells; others run the fused
-// kernel.
+// forces on designs of up to kGateJitMaxCells cells; others run the flat or the
+// fused kernel.
 #pragma once
 
 #include <cuda_runtime.h>

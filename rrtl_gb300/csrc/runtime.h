@@ -191,13 +191,20 @@ WordRunDev word_chunk_desc(const WordPrepared& g, uint64_t c0, uint64_t n, bool 
 // kept per design), or nullptr when the design or run does not qualify.
 const JitKernel* gate_jit_for_run(rrtl_design* d, const GateRunTables& t, uint32_t words);
 constexpr uint32_t kTunedCompiled = 0xFFFFFFFFu;
-// Designs whose peak of live nets (the fused program's slot count) is at
-// most this use the compiled gate kernel unless tuned otherwise: beyond it
-// the nets no longer fit the registers of one thread and spill.
+// The compiled gate kernel runs faster than the flat one wherever both were
+// timed (us a cycle with a hash, compiled / flat: 600 gates in 6 levels 0.66 /
+// 2.1 at 64 lanes and 1.2 / 11.5 at 262,144; 1,500 in 10 levels 1.6 / 2.3 and
+// 2.7 / 15.2; 3,000 in 100 levels 3.5 / 9.8 and 5.5 / 111; 8,000 in 160 levels
+// 16.0 / 16.5 at 64), but it is compiled for each set of run tables: the first run takes
+// 0.4 s at 150 gates, 0.7 at 600, 2.5 at 1,500, 8.6 at 3,000 and 55 at 8,000,
+// where the flat kernel's first run takes milliseconds. Unless the autotuner
+// measured otherwise, these designs use it without being asked:
+// designs whose peak of live nets (the fused program's slot count) is at most
+// this, which are small and whose nets fit the registers of one thread;
 constexpr uint32_t kGateJitAutoSlots = 192;
-// Designs of narrow levels (fewer cells per level on average than this) use
-// it too: the fused kernel's per-level barrier then dominates and most of its
-// warps idle, which costs more than spilled nets.
+// and designs of narrow levels (fewer cells per level on average than this),
+// where the flat kernel's level chain weighs most (16-bit ALU planes, 646 cells
+// in 65 levels: 0.78 / 4.4 at 64 lanes, 1.4 / 45 at 262,144).
 constexpr uint32_t kGateJitNarrowLevel = 48;
 // Host-side preparation a run of `lanes` lanes will need (the gate
 // program variant of its tile width, or the word kernel compiled for its
