@@ -87,4 +87,16 @@ struct FlatOptions {
 
 FlatProgram build_flat_program(const GateProgram& gp, uint32_t V, const FlatOptions& opt = {});
 
+// A shape of the flat kernel: row width V (0: none), vectors per warp set N,
+// warp sets Q.
+struct FlatShape {
+  uint32_t V = 0, N = 1, Q = 1;
+  bool narrow = false;  // on the kFlatNarrow program
+  uint32_t words() const { return V * N * Q; }
+};
+
+// Clocks of one tile-cycle, from the statistics of the program built for row
+// width `base`.
+double flat_tile_cost(const FlatProgram& fp, uint32_t base, const FlatShape& x);
+
 }  // namespace rrtl

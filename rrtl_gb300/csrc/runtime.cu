@@ -432,35 +432,11 @@ uint32_t choose_tile_words(rrtl_design* d, uint32_t words) {
 // Row width V, vectors per warp set N and warp sets Q of a flat run over
 // `words` 32-lane words (V = 0: the design does not fit), or those of an
 // explicit tile width. RRTL_FLAT=0 keeps the fused kernel and RRTL_FLAT=VNQ
-// forces a shape (A/B switches).
-//
-// A tile-cycle costs a boundary (stimulus, record, two barriers), a part per
-// level, one per entry and, in wide tiles, one per vector and its wavefronts.
-// Clocks, fitted to one wave of tiles on ten netlists of 3,000 to 200,000 gates
-// and 11 to 158 levels; the fit is within 8% of every one- and two-word tile
-// and 11% of every wider one (without the boundary: 41%, too low at 11 levels).
-// Measured, clocks a tile-cycle at 10,000 gates and 11 / 41 / 155 levels and at
-// 50,000 and 200,000 gates and 41 levels: one word 7.4k / 12.1k / 34.8k / 23.4k /
-// 58.9k (in the queue, 16 warps: 7.4k / 11.8k / 34.1k / 24.9k / 66.9k), two
-// 9.1k / 13.7k / 36.9k / 27.9k / 74.3k (8.9k / 13.7k / 36.7k / 29.3k / 80.9k),
-// one 4-word vector 10.9k / 17.5k / 44.5k / 36.6k / 105k, two 16.1k / 25.2k /
-// 56.8k / 56.2k, three 21.2k / 32.5k / 77.1k / 76.5k, four as two warp sets of
-// two 22.0k / 36.9k / 77.9k / 95.8k. Wide tiles pay until SMs are left without
-// one.
+// forces a shape (A/B switches). Wide tiles pay until SMs are left without one.
 constexpr FlatShape kFlatShapes[] = {{4, 2, 2}, {4, 3, 1}, {4, 2, 1}, {4, 1, 1}, {2, 1, 1}, {1, 1, 1}};
 // The tile width a flat run reports: several tiles of the widest documented
 // width that divides its own.
 uint32_t flat_reported_words(uint32_t w) { return w == 16 ? 8 : w == 12 ? 4 : w; }
-
-// Clocks of one tile-cycle, from the statistics of the program built for row
-// width `base`.
-double flat_tile_cost(const FlatProgram& fp, uint32_t base, const FlatShape& x) {
-  const double L = fp.n_levels, E = fp.n_entries;
-  if (x.V == 1) return x.narrow ? 3060.0 + 162.0 * L + 15.1 * E : 2880.0 + 147.0 * L + 17.4 * E;
-  if (x.V == 2) return x.narrow ? 3800.0 + 157.0 * L + 19.7 * E : 3550.0 + 159.0 * L + 21.2 * E;
-  const double vec4 = (double)fp.wavefronts * (base == 4 ? 1.0 : base == 2 ? 1.9 : 3.6);  // wavefronts of 4-word rows
-  return 3280.0 + 158.0 * L + 8.3 * E + x.N * x.Q * (935.0 + 49.0 * L + 1.06 * vec4);
-}
 
 // The widest rows that fit (0: none); packing leaves fewer live nets than the
 // fused program's slots.

@@ -84,14 +84,6 @@ struct FlatVariant {
   DevBuf d_stream, d_stream_net, d_warps, d_src_net, d_src_slot, d_commit;
 };
 
-// A shape of the flat kernel: row width V (0: none), vectors per warp set N,
-// warp sets Q.
-struct FlatShape {
-  uint32_t V = 0, N = 1, Q = 1;
-  bool narrow = false;  // on the kFlatNarrow program
-  uint32_t words() const { return V * N * Q; }
-};
-
 // Per-tile, per-stage force table of a batch for one tile width.
 struct ForceTable {
   bool valid = false;
