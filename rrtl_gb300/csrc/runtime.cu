@@ -478,8 +478,8 @@ FlatShape choose_flat(rrtl_design* d, uint32_t words, uint64_t cycles, uint32_t 
     if (x.V > top || (x.V == 4 && x.N * x.Q > v->max_n)) continue;
     if (tuned_w && flat_reported_words(x.words()) != tuned_w) continue;
     // Tiles past one a SM are split between blocks: no last round, but a split
-    // tile is loaded and stored once more, up to two tile-cycles a run (172
-    // one-word tiles on 152 SMs: 1.1 to 2.4 on the netlists above).
+    // tile is loaded and stored once more, about two tile-cycles a run (172
+    // one-word tiles on 152 SMs: 0.8 to 2.4 on netlists of 2,000 to 200,000 gates).
     const uint32_t tiles = (words + x.words() - 1) / x.words(), sms = d->ctx->sm_count;
     const double split = tiles > sms && tiles % sms ? 2.0 / (double)cycles : 0.0;
     const double t = (std::max(1.0, (double)tiles / sms) + split) * flat_tile_cost(v->fp, top, x);
